@@ -91,10 +91,10 @@ GRT_DEV Rhs7 ks_rhs(double x, double y, double z, double pt, double px, double p
     const double dB2 = 2.0 * r * dr2;
     const double dl01 = ((dr0 * x + r) - l1 * dB0) / B;
     const double dl02 = ((dr0 * y - a) - l2 * dB0) / B;
-    const double dl03 = (0.0 - l3 * dr0) / r;
+    const double dl03 = -(l3 * dr0) / r;
     const double dl11 = ((dr1 * x + a) - l1 * dB1) / B;
     const double dl12 = ((dr1 * y + r) - l2 * dB1) / B;
-    const double dl13 = (0.0 - l3 * dr1) / r;
+    const double dl13 = -(l3 * dr1) / r;
     const double dl21 = (dr2 * x - l1 * dB2) / B;
     const double dl22 = (dr2 * y - l2 * dB2) / B;
     const double dl23 = (1.0 - l3 * dr2) / r;
@@ -191,10 +191,10 @@ GRT_DEV Rhs7 ks_rhs_rcp(double x, double y, double z, double pt, double px, doub
     const double dB2 = 2.0 * r * dr2;
     const double dl01 = div_by((dr0 * x + r) - l1 * dB0, B, yB);
     const double dl02 = div_by((dr0 * y - a) - l2 * dB0, B, yB);
-    const double dl03 = div_by(0.0 - l3 * dr0, r, yr);
+    const double dl03 = div_by(-(l3 * dr0), r, yr);
     const double dl11 = div_by((dr1 * x + a) - l1 * dB1, B, yB);
     const double dl12 = div_by((dr1 * y + r) - l2 * dB1, B, yB);
-    const double dl13 = div_by(0.0 - l3 * dr1, r, yr);
+    const double dl13 = div_by(-(l3 * dr1), r, yr);
     const double dl21 = div_by(dr2 * x - l1 * dB2, B, yB);
     const double dl22 = div_by(dr2 * y - l2 * dB2, B, yB);
     const double dl23 = div_by(1.0 - l3 * dr2, r, yr);

@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(128, 4) trace_noalloc(const __grid_constant__ 
     grt::dev::Axes ax;
     grt::dev::KStore kk;
     grt::dev::stage_grid(kp, smem, INTEGRATOR, ax, kk);
-    grt::dev::trace_body<INTEGRATOR, grt::dev::Fp64Rhs, true>(kp, ax, kk);
+    grt::dev::trace_body<INTEGRATOR, grt::dev::Fp64RhsT<>, true>(kp, ax, kk);
 }
 
 grt_status set_err(char* err, size_t len, const char* msg) {

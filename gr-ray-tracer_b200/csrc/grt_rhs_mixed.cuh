@@ -44,9 +44,9 @@ static __device__ __noinline__ double renorm_alpha_ieee(double Bq, double disc, 
     return (-Bq + sqrt(disc)) / (2.0 * A);
 }
 
-// BF: the FP64 part is Fp64RhsT<BF>.  LAT: as for Fp64RhsT; the
-// renormalisation also takes the branch-free forms there.
-template <bool BF, bool LAT = false>
+// LAT: as for Fp64RhsT, the FP64 part; the renormalisation also takes the
+// branch-free forms there.
+template <bool LAT = false>
 struct MixedRhsT {
     static constexpr bool kLatency = LAT;
     static GRT_DEV V7 eval(const double s[8], const KParams& kp, int fast) {
@@ -54,7 +54,7 @@ struct MixedRhsT {
         const double rho2 = x * x + y * y;
         const double rsq = rho2 + z * z;
         if (!fast || rsq < kp.fp64_radius_sq || rho2 < kp.fp64_axis_sin2 * rsq)
-            return Fp64RhsT<BF, LAT>::eval(s, kp, 0);
+            return Fp64RhsT<LAT>::eval(s, kp, 0);
         return to_v7(ks_rhs_fp32(x, y, z, rsq, s[4], s[5], s[6], s[7], kp.a, kp.M));
     }
 
@@ -114,7 +114,6 @@ struct MixedRhsT {
         return r;
     }
 };
-using MixedRhs = MixedRhsT<false>;
 
 }  // namespace dev
 }  // namespace grt

@@ -1,7 +1,7 @@
 // Device self-checks of the reciprocal quotients of the FP64 right-hand side,
 // built into lib/libgrt_selftest.so (test infrastructure; the product library
 // does not link it), with -fmad=false like the trace kernels.
-//   grt_selftest_division  div_by(a, b, RN(1/b)) and IEEE a / b on the same operands;
+//   grt_selftest_division  div_by(+-a, |b|, RN(1/|b|)) and IEEE a / b on the same operands;
 //   grt_selftest_rhs       ks_rhs_rcp (and its box flag) and ks_rhs on the same states;
 //   grt_selftest_pow_quarter  the RK45 controller's pow_quarter on the device;
 //   grt_selftest_rn_box    the branch-free reciprocal and square root (grt_rn.cuh)
@@ -18,7 +18,9 @@ namespace {
 __global__ void division_kernel(const double* a, const double* b, size_t n, double* q_rcp, double* q_ieee) {
     const size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
     if (i >= n) return;
-    q_rcp[i] = grt::dev::div_by(a[i], b[i], grt::dev::div_recip(b[i]));
+    // div_by takes positive denominators: the sign of b goes to the numerator
+    const double den = fabs(b[i]), num = signbit(b[i]) ? -a[i] : a[i];
+    q_rcp[i] = grt::dev::div_by(num, den, grt::dev::div_recip(den));
     q_ieee[i] = a[i] / b[i];
 }
 
@@ -97,7 +99,7 @@ struct Bufs {
 
 extern "C" {
 
-// q_rcp[i] = div_by(a[i], b[i], RN(1/b[i])), q_ieee[i] = a[i] / b[i]; host
+// q_rcp[i] = div_by on |b[i]| with b[i]'s sign on a[i], q_ieee[i] = a[i] / b[i]; host
 // arrays of n values.  Returns a cudaError_t.
 int grt_selftest_division(const double* a, const double* b, size_t n, double* q_rcp, double* q_ieee) {
     if (n == 0) return 0;

@@ -58,24 +58,24 @@ static __device__ __noinline__ Rhs7 ks_rhs_ieee(double x, double y, double z, do
 }
 
 // Right-hand-side policy of the FP64 parity form: ks_rhs_rcp (reciprocal
-// quotients that round like IEEE divisions) inside its box, ks_rhs outside;
-// both give ks_rhs's result bit for bit.  BF: ks_rhs_rcp with the branch-free
-// reciprocal and square root (grt_rn.cuh), which a lone warp per scheduler
-// runs faster (C1's 4,096 rays: 3% on the trace) and the disk-mode kernel,
-// at 170 registers, slower (2%); the image-mode kernels use it.
+// quotients that round like IEEE divisions, with the branch-free reciprocal and
+// square root of grt_rn.cuh) inside its box, ks_rhs outside; both give ks_rhs's
+// result bit for bit.  Every kernel takes the branch-free functions: against
+// CUDA's they measured 3% faster on a trace of one warp per scheduler (4,096
+// RK4 rays) and 2.4% on the disk-mode transport (2.1e6 packets, 73.8 to 72.0 ms).
 // LAT: the instantiation is latency-bound (one warp or so per scheduler: the
 // 2-blocks/SM kernels), where the mixed form's renormalisation with the
 // branch-free functions and the branch-free Kerr-Schild radius (ks_radius_bf)
 // measured 4.6% faster on C1; at 4 blocks/SM and 128 registers the radius
 // measured 1% slower, so the others keep ks_radius.
 // `fast` is the per-call precision hint of the mixed form (ignored here).
-template <bool BF, bool LAT = false>
+template <bool LAT = false>
 struct Fp64RhsT {
     static constexpr bool kLatency = LAT;
     static GRT_DEV V7 eval(const double s[8], const KParams& kp, int /*fast*/) {
         if (kp.rcp_ok) {
             bool ok;
-            const Rhs7 o = ks_rhs_rcp<BF>(s[1], s[2], s[3], s[4], s[5], s[6], s[7], kp.a, kp.M, ok);
+            const Rhs7 o = ks_rhs_rcp<true>(s[1], s[2], s[3], s[4], s[5], s[6], s[7], kp.a, kp.M, ok);
             if (ok) return to_v7(o);
         }
         return to_v7(ks_rhs_ieee(s[1], s[2], s[3], s[4], s[5], s[6], s[7], kp.a, kp.M));
@@ -83,7 +83,6 @@ struct Fp64RhsT {
     // nothing to do after an accepted step; no radius computed (-1)
     static GRT_DEV double after_accept(double*, const KParams&, int) { return -1.0; }
 };
-using Fp64Rhs = Fp64RhsT<false>;
 
 struct Lane {
     double s[8];

@@ -12,19 +12,15 @@
 #include "grt_launch.h"
 #include "grt_trace.cuh"
 
-// The image-mode legs take the branch-free reciprocal and square root in the
-// FP64 right-hand side (dev::Fp64RhsT<true>); the disk-mode kernel measured
-// slower with them and keeps CUDA's.
-#define GRT_RHS_BF (GRT_LEG != 3)
 // The 2-blocks/SM kernels (255 registers; the workloads with about one warp
 // per scheduler) are latency-bound: their policies take LAT (grt_trace.cuh).
 #if GRT_MIXED
 #include "grt_rhs_mixed.cuh"
 #define GRT_TRACE_KERNEL trace_mixed
-#define GRT_TRACE_RHS(MINB) dev::MixedRhsT<GRT_RHS_BF, (MINB) == 2>
+#define GRT_TRACE_RHS(MINB) dev::MixedRhsT<(MINB) == 2>
 #else
 #define GRT_TRACE_KERNEL trace_fp64
-#define GRT_TRACE_RHS(MINB) dev::Fp64RhsT<GRT_RHS_BF, (MINB) == 2>
+#define GRT_TRACE_RHS(MINB) dev::Fp64RhsT<(MINB) == 2>
 #endif
 #define GRT_CAT2(a, b) a##b
 #define GRT_CAT(a, b) GRT_CAT2(a, b)
