@@ -153,6 +153,7 @@ struct grt_ctx {
     DevBuf<unsigned long long> scratch_u64;
     unsigned long long* host_u64 = nullptr;  // pinned
     grt_launch_config lc{128, 0, 8, 32, 1, 0, 0};
+    bool lc_set = false;  // the caller chose a launch shape (grt_set_launch_config)
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // images of the last grt_init_image_photons (one, cameras from p) or
     // grt_init_image_batch call; image k owns photon slots
@@ -337,7 +338,7 @@ grt::KParams make_kparams(const grt_ctx* c) {
                                 : (c->order_ph_ok ? c->order_ph.ptr : nullptr);
     k.calls_carry = c->calls_carry.ptr;
     k.counters = c->counters.ptr;
-    k.refill_threshold = c->lc.refill_threshold;
+    k.refill_threshold = c->lc_set ? c->lc.refill_threshold : grt::default_refill(k.image_mode);
     k.grab = c->lc.photons_per_grab;
     k.fp64_radius_sq = 16.0 * p.mass * p.mass + p.spin * p.spin;
     k.fp64_axis_sin2 = 0.01;
@@ -484,6 +485,7 @@ grt_status grt_set_launch_config(grt_ctx* c, const grt_launch_config* cfg) {
     if (cfg->max_iterations < 0) return fail(c, GRT_EINVAL, "max_iterations must be >= 0 (0 = automatic)");
     c->lc = *cfg;
     c->lc.pad = 0;
+    c->lc_set = true;
     ++c->generation;
     return GRT_OK;
 }

@@ -158,7 +158,9 @@ typedef struct grt_image_products {
 } grt_image_products;
 
 /* Launch shape of the trace kernel: the library's default is {128, 0, 8, 32, 1, 0, 0};
- * grt/autotune.py times the candidates on a workload and picks one. */
+ * grt/autotune.py times the candidates on a workload and picks one.  Until a shape is
+ * set (grt_set_launch_config) the refill threshold goes by the mode: 32 (whole tiles)
+ * in image mode, 4 in disk mode.  The shape never changes results. */
 typedef struct grt_launch_config {
     int32_t threads_per_block;    /* 128 (the trace kernels' block size) */
     int32_t blocks_per_sm;        /* 2, 3 or 4 resident blocks per SM: register caps 255 / 170 / 128;
