@@ -136,6 +136,8 @@ struct grt_ctx {
     bool separable = false;
     int nr = 0, nth = 0, nph = 0;
     double r_reject_lo = 0.0, r_reject_hi = 0.0;
+    grt::KGrid lookup{};                   // FP32 lookup constants and r_certain of the grid,
+    double lookup_spin = 0.0, lookup_mass = 0.0;  // the latter for this hole
     DevBuf<double> r_axis, th_axis, ph_axis, r_half, th_half, ph_half, r3, th3, ph3;
     DevBuf<double2> rho_t, vel, mag;
     DevBuf<double> cell_pos;               // [ncell][3] Cartesian KS cell positions (disk emission)
@@ -314,6 +316,11 @@ grt::KParams make_kparams(const grt_ctx* c) {
     g.mag = c->mag.ptr;
     g.r_reject_lo = c->r_reject_lo;
     g.r_reject_hi = c->r_reject_hi;
+    std::memcpy(g.origin, c->lookup.origin, sizeof(g.origin));
+    std::memcpy(g.per, c->lookup.per, sizeof(g.per));
+    std::memcpy(g.margin, c->lookup.margin, sizeof(g.margin));
+    g.even = c->lookup.even;
+    g.r_certain = p.spin == c->lookup_spin && p.mass == c->lookup_mass ? c->lookup.r_certain : INFINITY;
     k.m_abs = c->has_m_abs ? c->m_abs.ptr : nullptr;
     k.m_emis = c->has_m_emis ? c->m_emis.ptr : nullptr;
     if (c->batched) {
@@ -501,6 +508,7 @@ grt_status grt_upload_grid(grt_ctx* c, size_t nr, size_t nth, size_t nph, const 
     c->fluid_available = false;
     c->separable = false;
     c->nr = c->nth = c->nph = 0;
+    c->lookup = grt::KGrid{};
     if (ncell == 0) return GRT_OK;  // vacuum: fluid_available stays false
     if (!r || !th || !ph || !rho || !T || !vel4 || !mag4) return fail(c, GRT_EINVAL, "null grid array");
     if (nr > (1u << 30) || nth > (1u << 30) || nph > (1u << 30) || ncell > (1ull << 31))
@@ -565,8 +573,9 @@ grt_status grt_upload_grid(grt_ctx* c, size_t nr, size_t nth, size_t nph, const 
     GRT_CUDA(c, cudaMemcpy(c->r_axis.ptr, ra.data(), nr * sizeof(double), cudaMemcpyHostToDevice), "H2D axis");
     GRT_CUDA(c, cudaMemcpy(c->th_axis.ptr, ta.data(), nth * sizeof(double), cudaMemcpyHostToDevice), "H2D axis");
     GRT_CUDA(c, cudaMemcpy(c->ph_axis.ptr, pa.data(), nph * sizeof(double), cudaMemcpyHostToDevice), "H2D axis");
+    std::vector<double> rh(nr);
     if (sep) {
-        std::vector<double> rh(nr), th_h(nth), ph_h(nph);
+        std::vector<double> th_h(nth), ph_h(nph);
         grt::axes::half_spans(ra.data(), nr, 0, rh.data());
         grt::axes::half_spans(ta.data(), nth, 1, th_h.data());
         grt::axes::half_spans(pa.data(), nph, 2, ph_h.data());
@@ -584,6 +593,34 @@ grt_status grt_upload_grid(grt_ctx* c, size_t nr, size_t nth, size_t nph, const 
         GRT_CUDA(c, cudaMemcpy(c->r3.ptr, r, ncell * sizeof(double), cudaMemcpyHostToDevice), "H2D r3");
         GRT_CUDA(c, cudaMemcpy(c->th3.ptr, th, ncell * sizeof(double), cudaMemcpyHostToDevice), "H2D th3");
         GRT_CUDA(c, cudaMemcpy(c->ph3.ptr, ph, ncell * sizeof(double), cudaMemcpyHostToDevice), "H2D ph3");
+    }
+    c->lookup.nr = c->nr;
+    c->lookup.nth = c->nth;
+    c->lookup.nph = c->nph;
+    if (sep) grt::set_axis_lookup(c->lookup, ra.data(), ta.data(), pa.data());
+    c->lookup_spin = c->p.spin;
+    c->lookup_mass = c->p.mass;
+    c->lookup.r_certain = INFINITY;
+    if (sep) {
+        // the outermost shell with a cell whose tetrad is not certain, bounded
+        // over the cell: H <= M / r there, |l.u| <= |u0| + |u|
+        const size_t shell = nth * nph;
+        size_t i = nr;
+        while (i > 0) {
+            bool certain = true;
+            const double h2 = 2.0 * c->p.mass / (ra[i - 1] * std::exp(-rh[i - 1]));
+            for (size_t q = (i - 1) * shell; q < i * shell && certain; ++q) {
+                const double t2 = uv[2 * q].x * uv[2 * q].x;
+                const double s2 = uv[2 * q].y * uv[2 * q].y + uv[2 * q + 1].x * uv[2 * q + 1].x +
+                                  uv[2 * q + 1].y * uv[2 * q + 1].y;
+                const double lu = std::fabs(uv[2 * q].x) + std::sqrt(s2);
+                const double space = s2 + h2 * lu * lu;
+                certain = space - t2 < -1.0e-3 * (space + t2) && t2 < 1.0e300;
+            }
+            if (!certain) break;
+            --i;
+        }
+        if (i < nr) c->lookup.r_certain = i > 0 ? ra[i - 1] * std::exp(rh[i - 1]) * (1.0 + 1.0e-9) : 0.0;
     }
     c->fluid_available = true;
     return GRT_OK;

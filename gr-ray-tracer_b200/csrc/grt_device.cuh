@@ -93,15 +93,6 @@ GRT_DEV int bracket(const double* axis, int n, double q) {
     return lo;
 }
 
-GRT_DEV int nearest_radial_sorted(const double* r, int n, double radius) {
-    const int lo = bracket(r, n, radius);
-    if (lo < 0) return 0;
-    if (lo + 1 >= n) return lo;
-    const double dlo = fabs(log(radius / r[lo]));
-    const double dhi = fabs(log(radius / r[lo + 1]));
-    return dhi < dlo ? lo + 1 : lo;
-}
-
 GRT_DEV int nearest_polar_sorted(const double* th, int n, double polar) {
     const int lo = bracket(th, n, polar);
     if (lo < 0) return 0;
@@ -132,16 +123,11 @@ GRT_DEV int nearest_azimuth_sorted(const double* ph, int n, double az) {
     return c1 < c2 ? c1 : c2;
 }
 
-// scattering.hpp:99-149 on one separable axis, with the neighbour half-span
-// precomputed per axis value (see KGrid::r_half).
-GRT_DEV bool within_radial_sorted(const double* r, const double* half, int i, double radius) {
-    return fabs(log(radius / r[i])) <= half[i];
-}
-
-// nearest_radial_sorted and within_radial_sorted in one pass: the log
-// distance of the chosen cell is the one the nearest-cell test computed, so it
-// is evaluated once per candidate (one or two), through one site.  Ties go to
-// the lower index, as in nearest_radial_sorted.
+// The nearest radial cell and whether it accepts the radius (scattering.hpp:
+// 99-117 with the neighbour half-span precomputed per axis value, see
+// KGrid::r_half): the log distance of the chosen cell is the one the
+// nearest-cell test computed, so it is evaluated once per candidate (one or
+// two), through one site.  Ties go to the lower index.
 GRT_DEV bool locate_radial_sorted(const double* r, const double* half, int n, double radius, int& i) {
     const int lo = bracket(r, n, radius);
     const int c0 = lo < 0 ? 0 : lo;
@@ -269,6 +255,8 @@ struct FluidSample {
 };
 
 // fluid_frame.hpp:51-80 with the metric already evaluated at the photon.
+// UNROLL: as straight-line code, which disappears where its result is unused.
+template <bool UNROLL = false>
 GRT_DEV bool build_tetrad(const double g[4][4], const double u[4], double e[4][4]) {
     const double vn = metric_dot(g, u, u);
     if (!(vn < 0.0) || !isfinite(vn)) return false;
@@ -276,15 +264,14 @@ GRT_DEV bool build_tetrad(const double g[4][4], const double u[4], double e[4][4
     const double ts = u[0] >= 0.0 ? 1.0 : -1.0;
 #pragma unroll
     for (int mu = 0; mu < 4; ++mu) e[0][mu] = ts * u[mu] * inv;
-    // Rolled over the spatial axes (one square-root and one division site):
-    // the tetrad is built on every fluid sample, so its code stays small.
-#pragma unroll 1
+    // Rolled over the spatial axes (one square-root and one division site).
+#pragma unroll(UNROLL ? 3 : 1)
     for (int axis = 0; axis < 3; ++axis) {
         double cand[4];
         const double tp = metric_dot_unit(g, e[0], axis + 1);
 #pragma unroll
         for (int mu = 0; mu < 4; ++mu) cand[mu] = (mu == axis + 1 ? 1.0 : 0.0) + tp * e[0][mu];
-#pragma unroll 1
+#pragma unroll(UNROLL ? 3 : 1)
         for (int prev = 0; prev < axis; ++prev) {
             const double proj = metric_dot(g, e[prev + 1], cand);
 #pragma unroll
@@ -299,11 +286,23 @@ GRT_DEV bool build_tetrad(const double g[4][4], const double u[4], double e[4][4
     return true;
 }
 
-// sample_scattering_fluid (scattering.hpp:185-251).  `radius` is
-// compute_r(x, y, z, spin) of the state, which the caller has already.
-// Cartesian velocity / magnetic four-vectors per cell are precomputed on the
-// host with the reference's transform (fluid_frame.hpp:28-48) and unit scale,
-// so the per-step arithmetic is exactly the reference's.
+// sample_scattering_fluid (scattering.hpp:185-251) in parts, so that a step
+// evaluates only what it uses:
+//   locate_fluid   the cell a position samples;
+//   fluid_cell     what the extension points receive, read from the cell;
+//   fluid_valid    whether the fluid tetrad exists there;
+//   full_sample    the cell with its tetrad and fluid-frame field (emission,
+//                  scattering: once per event).
+// Before, every in-grid step built the whole sample out of line -- the lookup
+// with its logarithms, the tetrad's four square roots and 25 metric products --
+// and passed it through local memory, though the default absorption and
+// emission read the density and temperature alone; a lone packet's call spent
+// about half of its 23,000 cycles on it.  In parts, with the FP32 lookup below,
+// on one B200: 64 images (4.76e6 rays) 40.2 to 35.5 ms, 65,536 rays 1.17 to 1.06,
+// the checkpointed forward of 16,384 rays 2.73 to 1.92, 1.1e5 disk packets 9.3
+// to 6.9 and, with trace_body's deferred scattering, 2.07e6 packets 62.4 to 47.2.
+// `radius` is compute_r(x, y, z, spin) of the state, which the caller has already.
+
 // fluid_frame.hpp:28-48 on the device, times the [units] scale (raw layout only).
 GRT_DEV void spherical_to_cartesian_scaled(double r, double th, double ph, double spin, const double* sv,
                                           double scale, double c[4]) {
@@ -322,9 +321,6 @@ GRT_DEV void spherical_to_cartesian_scaled(double r, double th, double ph, doubl
     c[3] = (radial_z * sv[1] + theta_z * sv[2]) * scale;
 }
 
-// RAW selects the grid layout: false -- packed (rho, T) pairs and Cartesian
-// four-vectors precomputed on the host; true -- the reference's raw arrays,
-// with the spherical-to-Cartesian conversion done per sample.
 // Separable axes and their half-spans staged in shared memory.
 struct Axes {
     const double* r;
@@ -335,78 +331,267 @@ struct Axes {
     const double* phh;
 };
 
-template <bool RAW>
-static __device__ __noinline__ bool sample_fluid_at(const KParams& kp, const Axes ax, double t, double x,
-                                                    double y, double z, double radius, FluidSample* outp) {
-    FluidSample& out = *outp;
-    const double s[4] = {t, x, y, z};
+// The reference's lookup (scattering.hpp:41-180) with its own arithmetic: the
+// cell index, or -1 outside every cell.
+static __device__ __noinline__ int locate_exact(const KParams& kp, const Axes ax, double x, double y, double z,
+                                                double radius) {
     const KGrid& G = kp.grid;
     int i, j, k;
     if (G.separable) {
-        if (!locate_radial_sorted(ax.r, ax.rh, G.nr, radius, i)) return false;
+        if (!locate_radial_sorted(ax.r, ax.rh, G.nr, radius, i)) return -1;
     }
-    const double ct = fmax(-1.0, fmin(1.0, s[3] / radius));
+    const double ct = fmax(-1.0, fmin(1.0, z / radius));
     const double polar = acos(ct);
-    double az = atan2(radius * s[2] - kp.a * s[1], radius * s[1] + kp.a * s[2]);
+    double az = atan2(radius * y - kp.a * x, radius * x + kp.a * y);
     if (az < 0.0) az += 2.0 * kPi;
     if (G.separable) {
         j = nearest_polar_sorted(ax.th, G.nth, polar);
         k = nearest_azimuth_sorted(ax.ph, G.nph, az);
-        if (!within_polar_sorted(ax.th, ax.thh, j, polar) || !within_azimuth_sorted(ax.ph, ax.phh, k, az))
-            return false;
+        if (!within_polar_sorted(ax.th, ax.thh, j, polar) || !within_azimuth_sorted(ax.ph, ax.phh, k, az)) return -1;
     } else {
         const Grid3 g3{G.r3, G.th3, G.ph3, G.nr, G.nth, G.nph};
-        if (!locate_general(g3, radius, polar, az, i, j, k)) return false;
+        if (!locate_general(g3, radius, polar, az, i, j, k)) return -1;
     }
-    const int cell = (i * G.nth + j) * G.nph + k;
-    out.cell = cell;
-    FluidCellCGS& f = out.fluid;
+    return (i * G.nth + j) * G.nph + k;
+}
+
+// The interval of a strictly increasing axis that holds q (axis[lo] <= q <
+// axis[lo + 1]) for axis[0] <= q < axis[n - 1]: `guess`, the interval on an
+// evenly spaced axis, when it does, else by search.
+GRT_DEV int bracket_from(const double* axis, int n, double q, int guess) {
+    guess = max(0, min(guess, n - 2));
+    if (axis[guess] <= q && q < axis[guess + 1]) return guess;
+    return bracket(axis, n, q);
+}
+
+// FP32 polar angle and azimuth of a position in Kerr-Schild coordinates:
+// tan(theta) = sin / cos with sin^2 = (x^2 + y^2) / (r^2 + a^2), cos = z / r.
+// For radii whose squares FP32 holds.
+constexpr double kFp32RadiusMin = 1.0e-12, kFp32RadiusMax = 1.0e12;
+GRT_DEV void angles_fp32(double a, double x, double y, double z, double r, float& th, float& az) {
+    const float rf = static_cast<float>(r), af = static_cast<float>(a);
+    th = atan2f(sqrtf(static_cast<float>(x * x + y * y)) * rf, static_cast<float>(z) * sqrtf(rf * rf + af * af));
+    az = atan2f(static_cast<float>(r * y - a * x), static_cast<float>(r * x + a * y));
+}
+
+// locate_exact's cell on a separable grid without its logarithms and inverse
+// trigonometric functions in double precision, or kUndecided: for axes of any
+// spacing.  The angles and
+// the logarithm are taken in FP32 (a few 1e-7 off, see kAngleMargin) and the
+// radius is compared through squares; a position within the margin of a
+// decision -- a midpoint between two cells, the end of a cell's acceptance --
+// is left to locate_exact, about one in a thousand on a 128 x 64 x 64 grid.
+// A position nearer to its cell's centre than the midpoint, by the margin, is
+// inside the cell's half-width: that is 0.500001 times the larger neighbour
+// gap.  Beyond the outermost centres the half-width itself decides.
+constexpr int kUndecided = -2;
+// Bound on the error of the FP32 angles: the arguments carry one rounding and
+// the square root, quotient and atan2f a few ulp each, together below 2e-6 at
+// 2 pi; five times that.  The FP32 logarithm of a ratio near 1 is far closer.
+constexpr double kAngleMargin = 1.0e-5;
+
+static __device__ __noinline__ int locate_stretched(const KGrid& G, const Axes ax, double a, double x, double y,
+                                                    double z, double r) {
+    if (!(r > kFp32RadiusMin && r < kFp32RadiusMax) || G.nr < 2 || G.nth < 2) return kUndecided;
+    // radius: nearest in the logarithm.  The logarithms' rounding is far
+    // inside the margins while the gap is above 1e-6.
+    int i;
+    if (r < ax.r[0] || r >= ax.r[G.nr - 1]) {
+        i = r < ax.r[0] ? 0 : G.nr - 1;
+        const double d = fabsf(logf(static_cast<float>(r / ax.r[i])));
+        if (!(fabs(d - ax.rh[i]) > kAngleMargin)) return kUndecided;
+        if (d > ax.rh[i]) return -1;
+    } else {
+        i = bracket_from(ax.r, G.nr, r, __float2int_rd((logf(static_cast<float>(r)) - G.origin[0]) * G.per[0]));
+        const double rlo = ax.r[i], rhi = ax.r[i + 1];
+        const double rr = r * r, mid = rlo * rhi;
+        if (!(rhi - rlo > 1.0e-6 * rlo) || !(fabs(rr - mid) > 0x1p-40 * mid)) return kUndecided;
+        if (rr > mid) ++i;
+    }
+    float thf, azf;
+    angles_fp32(a, x, y, z, r, thf, azf);
+    const double th = thf;
+    int j;
+    if (th < ax.th[0] || th >= ax.th[G.nth - 1]) {
+        j = th < ax.th[0] ? 0 : G.nth - 1;
+        const double d = fabs(th - ax.th[j]);
+        if (!(fabs(d - ax.thh[j]) > kAngleMargin)) return kUndecided;
+        if (d > ax.thh[j]) return -1;
+    } else {
+        j = bracket_from(ax.th, G.nth, th, __float2int_rd(static_cast<float>(th - ax.th[0]) * G.per[1]));
+        const double dth = (th - ax.th[j]) - (ax.th[j + 1] - th);
+        if (!(fabs(dth) > 2.0 * kAngleMargin)) return kUndecided;
+        if (dth > 0.0) ++j;
+    }
+    // azimuth: the neighbours on the circle
+    const double az = azf < 0.0f ? static_cast<double>(azf) + 2.0 * kPi : static_cast<double>(azf);
+    const int n = G.nph;
+    const double p0 = ax.ph[0], p1 = ax.ph[n - 1];
+    int k = n - 1, k2 = 0;
+    double d, d2;  // distances to the centres on either side
+    if (az < p0 || az >= p1) {
+        d = az - p1 + (az < p0 ? 2.0 * kPi : 0.0);
+        d2 = p0 - az + (az < p0 ? 0.0 : 2.0 * kPi);
+    } else {
+        k = bracket_from(ax.ph, n, az, __float2int_rd(static_cast<float>(az - p0) * G.per[2]));
+        k2 = k + 1;
+        d = az - ax.ph[k];
+        d2 = ax.ph[k2] - az;
+    }
+    // gaps of half the circle or more would make the other way round the shorter
+    if (!(d + d2 < 3.0) || !(fabs(d - d2) > 2.0 * kAngleMargin)) return kUndecided;
+    if (d2 < d) {
+        k = k2;
+        d = d2;
+    }
+    const double half = ax.phh[k];
+    if (!(fabs(d - half) > kAngleMargin)) return kUndecided;
+    if (d > half) return -1;
+    return (i * G.nth + j) * G.nph + k;
+}
+
+// The same on a grid that is even in log r, theta and phi, with phi all the
+// way round (KGrid::even; what the torus generators write): the cell is the
+// nearest integer to the position in units of the spacing, no axis is read
+// and no lane branches.  A position within KGrid::margin of a cell's edge --
+// the error of the FP32 angle or logarithm in that unit, and the evenness the
+// host asks of the axis -- is left to locate_exact; an edge cell ends within
+// 0.500001 of the spacing, so beyond the margin a position outside is outside.
+GRT_DEV int locate_even(const KGrid& G, double a, double x, double y, double z, double r) {
+    if (!(r > kFp32RadiusMin && r < kFp32RadiusMax)) return kUndecided;
+    float th, az;
+    angles_fp32(a, x, y, z, r, th, az);
+    if (az < 0.0f) az += 6.2831853f;
+    const float fi = (logf(static_cast<float>(r)) - G.origin[0]) * G.per[0];
+    const float fj = (th - G.origin[1]) * G.per[1], fk = (az - G.origin[2]) * G.per[2];
+    const float i = rintf(fi), j = rintf(fj), k = rintf(fk);
+    if (!(fabsf(fi - i) < G.margin[0] && fabsf(fj - j) < G.margin[1] && fabsf(fk - k) < G.margin[2])) return kUndecided;
+    if (i < 0.0f || i > static_cast<float>(G.nr - 1) || j < 0.0f || j > static_cast<float>(G.nth - 1)) return -1;
+    int kk = static_cast<int>(k);
+    kk += kk < 0 ? G.nph : kk >= G.nph ? -G.nph : 0;
+    return (static_cast<int>(i) * G.nth + static_cast<int>(j)) * G.nph + kk;
+}
+
+// The cell that samples a position, or -1: the cheap rejections first.
+GRT_DEV int locate_fluid(const KParams& kp, const Axes& ax, double x, double y, double z, double radius) {
+    const KGrid& G = kp.grid;
+    if (!G.available) return -1;
+    if (!(radius > 0.0) || !isfinite(radius)) return -1;
+    if (radius < G.r_reject_lo || radius > G.r_reject_hi) return -1;
+    int cell = kUndecided;
+    if (G.even) cell = locate_even(G, kp.a, x, y, z, radius);
+    else if (G.separable) cell = locate_stretched(G, ax, kp.a, x, y, z, radius);
+    if (cell == kUndecided) cell = locate_exact(kp, ax, x, y, z, radius);
+    return cell;
+}
+
+// The cell's CGS record at a position, but for the fluid-frame field.  Parts
+// that nothing reads are not loaded.
+// RAW selects the grid layout: false -- packed (rho, T) pairs and Cartesian
+// four-vectors precomputed on the host; true -- the reference's raw arrays,
+// with the spherical-to-Cartesian conversion done per sample.
+template <bool RAW>
+GRT_DEV void fluid_cell(const KParams& kp, int cell, const double s[4], FluidCellCGS& f) {
+    const KGrid& G = kp.grid;
     f.position_cm[0] = s[1] * kp.length_scale;
     f.position_cm[1] = s[2] * kp.length_scale;
     f.position_cm[2] = s[3] * kp.length_scale;
     f.coordinate_time_s = s[0] * kp.time_scale;
-    double cm[4];
     if (RAW) {
         f.density_g_cm3 = G.rho_raw[cell] * kp.density_scale;
         f.temperature_k = G.T_raw[cell] * kp.temperature_scale;
-        if (!(f.density_g_cm3 > 0.0) || !isfinite(f.density_g_cm3) || !isfinite(f.temperature_k))
-            return false;
         spherical_to_cartesian_scaled(G.r3[cell], G.th3[cell], G.ph3[cell], kp.a, G.vel_raw + 4 * cell,
                                       G.vel_scale, f.coordinate_four_velocity_cm_s);
-        spherical_to_cartesian_scaled(G.r3[cell], G.th3[cell], G.ph3[cell], kp.a, G.mag_raw + 4 * cell,
-                                      G.mag_scale, cm);
     } else {
         const double2 rt = G.rho_t[cell];
         f.density_g_cm3 = rt.x * kp.density_scale;
         f.temperature_k = rt.y * kp.temperature_scale;
-        if (!(f.density_g_cm3 > 0.0) || !isfinite(f.density_g_cm3) || !isfinite(f.temperature_k))
-            return false;
         const double2 u01 = G.vel[2 * cell], u23 = G.vel[2 * cell + 1];
         f.coordinate_four_velocity_cm_s[0] = u01.x;
         f.coordinate_four_velocity_cm_s[1] = u01.y;
         f.coordinate_four_velocity_cm_s[2] = u23.x;
         f.coordinate_four_velocity_cm_s[3] = u23.y;
+    }
+}
+
+GRT_DEV bool fluid_finite(const FluidCellCGS& f) {
+    return f.density_g_cm3 > 0.0 && isfinite(f.density_g_cm3) && isfinite(f.temperature_k);
+}
+
+// The tetrad at a position in `cell` (f from fluid_cell) and the fluid-frame
+// field in it; false where there is no tetrad.
+template <bool RAW, bool UNROLL = false>
+GRT_DEV bool fluid_frame(const KParams& kp, int cell, double x, double y, double z, double radius, FluidCellCGS& f,
+                         double e[4][4]) {
+    const KGrid& G = kp.grid;
+    double cm[4];
+    if (RAW) {
+        spherical_to_cartesian_scaled(G.r3[cell], G.th3[cell], G.ph3[cell], kp.a, G.mag_raw + 4 * cell,
+                                      G.mag_scale, cm);
+    } else {
         const double2 b01 = G.mag[2 * cell], b23 = G.mag[2 * cell + 1];
         cm[0] = b01.x; cm[1] = b01.y; cm[2] = b23.x; cm[3] = b23.y;
     }
     MetricAt m;
-    ks_metric_from_r(s[1], s[2], s[3], radius, kp.a, kp.M, m);
-    if (!build_tetrad(m.g, f.coordinate_four_velocity_cm_s, out.e)) return false;
-    f.magnetic_gauss[0] = -metric_dot(m.g, out.e[0], cm);
+    ks_metric_from_r(x, y, z, radius, kp.a, kp.M, m);
+    if (!build_tetrad<UNROLL>(m.g, f.coordinate_four_velocity_cm_s, e)) return false;
+    f.magnetic_gauss[0] = -metric_dot(m.g, e[0], cm);
 #pragma unroll
-    for (int axis = 1; axis < 4; ++axis) f.magnetic_gauss[axis] = metric_dot(m.g, out.e[axis], cm);
+    for (int axis = 1; axis < 4; ++axis) f.magnetic_gauss[axis] = metric_dot(m.g, e[axis], cm);
     return true;
 }
 
-// sample_scattering_fluid (scattering.hpp:185-251): the cheap early-outs
-// inline, the lookup + gather + tetrad out of line.
-template <bool RAW = false>
-GRT_DEV bool sample_fluid(const KParams& kp, const Axes& ax, const double s[8], double radius, FluidSample& out) {
-    const KGrid& G = kp.grid;
-    if (!G.available) return false;
-    if (!(radius > 0.0) || !isfinite(radius)) return false;
-    if (radius < G.r_reject_lo || radius > G.r_reject_hi) return false;
-    return sample_fluid_at<RAW>(kp, ax, s[0], s[1], s[2], s[3], radius, &out);
+// The whole sample of `cell` at a position; false where the density, the
+// temperature or the tetrad is not valid.
+template <bool RAW>
+static __device__ __noinline__ bool full_sample(const KParams& kp, int cell, double t, double x, double y, double z,
+                                                double radius, FluidSample* out) {
+    const double s[4] = {t, x, y, z};
+    out->cell = cell;
+    fluid_cell<RAW>(kp, cell, s, out->fluid);
+    return fluid_finite(out->fluid) && fluid_frame<RAW>(kp, cell, x, y, z, radius, out->fluid, out->e);
+}
+
+// full_sample's verdict alone.
+template <bool RAW>
+static __device__ __noinline__ bool full_sample_valid(const KParams& kp, int cell, double t, double x, double y,
+                                                      double z, double radius) {
+    FluidSample fs;
+    return full_sample<RAW>(kp, cell, t, x, y, z, radius, &fs);
+}
+
+// Whether the tetrad of four-velocity u exists at a position (build_tetrad's
+// verdict).  u.u = -u0^2 + |u|^2 + 2H (l.u)^2 here carries a few roundings of
+// its terms, so one that is negative by a thousandth of their sum is negative
+// in build_tetrad's arithmetic too; the normalised e0 then stays below 32, and
+// the norms that build_tetrad tests -- Schur complements of
+// delta_ij + 2H l_i l_j + e0_i e0_j, at least 1 -- keep nine digits.  Anything
+// closer to the light cone is left to build_tetrad itself.
+GRT_DEV bool tetrad_certain(double x, double y, double z, double r, double a, double M, const double u[4]) {
+    const double ar = a * a + r * r, az = a * z, r2 = r * r;
+    const double lu = u[0] + ((r * x + a * y) * u[1] + (r * y - a * x) * u[2]) * rcp_rn_box(ar) + z * u[3] * rcp_rn_box(r);
+    const double h = 2.0 * M * r2 * r * rcp_rn_box(r2 * r2 + az * az) * (lu * lu);
+    const double t2 = u[0] * u[0], s2 = u[1] * u[1] + u[2] * u[2] + u[3] * u[3] + h;
+    return s2 - t2 < -1.0e-3 * (s2 + t2) && t2 < 1.0e300 && r > 1.0e-6 && r < 1.0e30 && fabs(a) < 1.0e30;
+}
+
+// The fluid at a position, as the extension points and the scattering draw
+// receive it: the cell, or -1 when nothing is sampled (scattering.hpp:185-251's
+// false).  The fluid-frame field costs the whole tetrad; it is straight-line
+// code that the compiler drops while no extension point reads magnetic_gauss.
+template <bool RAW>
+GRT_DEV int sample_fluid(const KParams& kp, const Axes& ax, const double s[8], double radius, FluidCellCGS& f) {
+    const int cell = locate_fluid(kp, ax, s[1], s[2], s[3], radius);
+    if (cell < 0) return -1;
+    fluid_cell<RAW>(kp, cell, s, f);
+    if (!fluid_finite(f)) return -1;
+    if (!(radius > kp.grid.r_certain) &&
+        !tetrad_certain(s[1], s[2], s[3], radius, kp.a, kp.M, f.coordinate_four_velocity_cm_s) &&
+        !full_sample_valid<RAW>(kp, cell, s[0], s[1], s[2], s[3], radius))
+        return -1;
+    double e[4][4];
+    fluid_frame<RAW, true>(kp, cell, s[1], s[2], s[3], radius, f, e);
+    return cell;
 }
 
 // ---------------------------------------------------------------------------
@@ -426,25 +611,37 @@ struct ScatterState {
 // maybe_scatter_photon (scattering.hpp:259-313) in two parts.  scatter_drawn is the
 // part every sampled step takes, inline: the Thomson optical depth over the
 // proposed step and the first draw; it says whether the packet scatters.
-GRT_DEV bool scatter_drawn(double dl, double length_scale, const FluidSample& fs, Philox& rng) {
+GRT_DEV bool scatter_drawn(double dl, double length_scale, const FluidCellCGS& fluid, Philox& rng) {
     const double path_cm = dl * length_scale;
-    const double ne = fs.fluid.density_g_cm3 / kProtonMassCgs;
+    const double ne = fluid.density_g_cm3 / kProtonMassCgs;
     const double tau = kSigmaThomsonCgs * ne * path_cm;
     const double prob = 1.0 - exp(-tau);
     return !(rng.drand() >= prob);  // the reference's rejection test, NaN included
 }
 
-// The rest, out of line and only for a packet that scatters: the isotropic
+// The rest, out of line and only for a packet that scatters: the tetrad of its
+// cell (which exists: the step sampled it), the isotropic
 // fluid-frame direction (two more draws), the new covariant momentum and the
-// albedo weights; false leaves the state as it was.
-static __device__ __noinline__ bool scatter_packet(ScatterState* st, double albedo, const FluidSample& fs, double a,
-                                                   double M, Philox* rngp) {
-    Philox& rng = *rngp;
+// albedo weights; false leaves the state as it was.  The stream of (photon,
+// step) is opened again and scatter_drawn's draw passed over, so that no
+// generator state waits with the packet.
+template <bool RAW>
+static __device__ __noinline__ bool scatter_packet(const KParams& kp, ScatterState* st, int cell, double radius,
+                                                   uint64_t id, int64_t step) {
+    Philox rng(kp.seed, id, static_cast<uint32_t>(step));
+    rng.drand();
     double* s = st->s;
     double* I = st->I;
+    const double albedo = kp.albedo;
+    FluidCellCGS f;
+    fluid_cell<RAW>(kp, cell, s, f);
+    MetricAt m;
+    ks_metric_from_r(s[1], s[2], s[3], radius, kp.a, kp.M, m);
+    double e[4][4];
+    build_tetrad<true>(m.g, f.coordinate_four_velocity_cm_s, e);
     double E = 0.0;
 #pragma unroll
-    for (int mu = 0; mu < 4; ++mu) E -= s[4 + mu] * fs.e[0][mu];
+    for (int mu = 0; mu < 4; ++mu) E -= s[4 + mu] * e[0][mu];
     if (!(E > 0.0) || !isfinite(E)) return false;
     const double mu_c = 2.0 * rng.drand() - 1.0;
     const double dphi = 2.0 * kPi * rng.drand();
@@ -454,9 +651,7 @@ static __device__ __noinline__ bool scatter_packet(ScatterState* st, double albe
     const double dx = tr * cs, dy = tr * sn, dz = mu_c;
     double w[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) w[q] = fs.e[0][q] + dx * fs.e[1][q] + dy * fs.e[2][q] + dz * fs.e[3][q];
-    MetricAt m;
-    ks_metric(s[1], s[2], s[3], a, M, m);
+    for (int q = 0; q < 4; ++q) w[q] = e[0][q] + dx * e[1][q] + dy * e[2][q] + dz * e[3][q];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         double pq = 0.0;

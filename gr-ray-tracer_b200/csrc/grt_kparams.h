@@ -29,6 +29,12 @@ struct KGrid {
     const double2* rho_t;   // [ncells] (rho, T) in code units
     const double2* vel;     // [2*ncells] Cartesian KS u^mu * velocity scale
     const double2* mag;     // [2*ncells] Cartesian KS b^mu * magnetic scale
+    // separable axes in units of their spacing, in log r, theta, phi: cell 0,
+    // cells per unit, and how far from a cell's centre the FP32 lookup decides
+    // (locate_even; with even = 0 only an index guess, locate_stretched)
+    float origin[3], per[3], margin[3];
+    int even;
+    double r_certain;       // every cell sampled beyond it has a tetrad (tetrad_certain)
     double r_reject_lo;     // radii outside [lo, hi] cannot pass within_radial_cell
     double r_reject_hi;
     // Raw reference layout (allocation-free entry point): the seven arrays as

@@ -150,6 +150,33 @@ inline int rcp_params_ok(double a, double M) {
     return a_ok && m_ok ? 1 : 0;
 }
 
+// The FP32 lookup's constants from the host's copy of separable axes.  Even:
+// every value within 1e-6 of its place in units of the spacing, phi all the
+// way round.  The FP32 error (4e-6 bounds angle, logarithm and its rounding
+// in [0, 2 pi]; the logarithm's grows with its size) must stay below a
+// hundredth of the spacing, and is taken five times over.
+inline void set_axis_lookup(KGrid& g, const double* ra, const double* ta, const double* pa) {
+    const double* axes[3] = {ra, ta, pa};
+    const int n[3] = {g.nr, g.nth, g.nph};
+    bool even = true;
+    for (int q = 0; q < 3; ++q) {
+        auto at = [&](int i) { return q == 0 ? std::log(axes[q][i]) : axes[q][i]; };
+        const double lo = at(0), hi = at(n[q] - 1);
+        const double per = n[q] > 1 && hi > lo ? (n[q] - 1) / (hi - lo) : 0.0;
+        double err = 4.0e-6 * per;
+        if (q == 0) err = (1.0e-6 + 3.0e-7 * std::fmax(std::fabs(lo), std::fabs(hi))) * per;
+        g.origin[q] = static_cast<float>(lo);
+        g.per[q] = static_cast<float>(per);
+        // the float product is itself rounded: an index of n carries n 2^-23
+        err = 5.0 * (err + 2.0e-6 + n[q] * 2.4e-7);
+        g.margin[q] = static_cast<float>(0.5 - err);
+        even = even && per > 0.0 && err < 0.05;
+        if (q == 2) even = even && std::fabs(n[q] - per * 6.283185307179586) < 1.0e-6;
+        for (int i = 0; i < n[q] && even; ++i) even = std::fabs((at(i) - lo) * per - i) < 1.0e-6;
+    }
+    g.even = even ? 1 : 0;
+}
+
 // Dynamic shared memory of a trace launch: the stage slots for RK45 (6*7
 // doubles per thread: k1..k5, then the state) plus the separable axes and
 // their half-spans (2*(nr+nth+nph)).

@@ -190,6 +190,10 @@ extern "C" grt_status grt_trace_device_noalloc(const grt_params* p, const grt_de
             grt::axes::half_spans(ta, nth, 1, hh + nr);
             grt::axes::half_spans(pa, nph, 2, hh + nr + nth);
             grt::axes::radial_reject_bounds(ra, nr, &gm.r_reject_lo, &gm.r_reject_hi);
+            kp.grid.nr = static_cast<int>(nr);
+            kp.grid.nth = static_cast<int>(nth);
+            kp.grid.nph = static_cast<int>(nph);
+            grt::set_axis_lookup(kp.grid, ra, ta, pa);
             // returns once the pageable source is staged, so the buffer may be
             // reused after the lock is released
             e = cudaMemcpyAsync(axes + nax, hh, nax * sizeof(double), cudaMemcpyHostToDevice, stream);
@@ -247,6 +251,7 @@ extern "C" grt_status grt_trace_device_noalloc(const grt_params* p, const grt_de
         g.vel_raw = grid->vel4;
         g.mag_raw = grid->mag4;
     }
+    g.r_certain = INFINITY;
     g.vel_scale = p->four_velocity_cm_s_per_code;
     g.mag_scale = p->magnetic_gauss_per_code;
     g.r_reject_lo = gm.r_reject_lo;

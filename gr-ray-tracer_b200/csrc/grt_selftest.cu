@@ -6,11 +6,17 @@
 //   grt_selftest_pow_quarter  the RK45 controller's pow_quarter on the device;
 //   grt_selftest_rn_box    the branch-free reciprocal and square root (grt_rn.cuh)
 //                          and CUDA's __drcp_rn and sqrt on the same arguments;
-//   grt_selftest_rhs_bf    ks_rhs_rcp with the branch-free functions and with CUDA's.
+//   grt_selftest_rhs_bf    ks_rhs_rcp with the branch-free functions and with CUDA's;
+//   grt_selftest_locate    the FP32 cell lookups and the reference's on the same positions;
+//   grt_selftest_tetrad    tetrad_certain and build_tetrad on the same four-velocities.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include "grt_metric.cuh"
+#include <vector>
+
+#include "grt_device.cuh"
+#include "grt_grid_axes.h"
+#include "grt_launch.h"
 #include "grt_pow_quarter.cuh"
 
 namespace {
@@ -72,6 +78,30 @@ __global__ void pow_quarter_kernel(const double* x, size_t n, double* y) {
     const size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
     if (i >= n) return;
     y[i] = grt::pow_quarter(x[i]);
+}
+
+__global__ void locate_kernel(const __grid_constant__ grt::KParams kp, grt::dev::Axes ax, const double* pos, size_t n,
+                              int* even, int* stretched, int* exact) {
+    const size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
+    if (i >= n) return;
+    const double x = pos[3 * i], y = pos[3 * i + 1], z = pos[3 * i + 2];
+    const double r = grt::dev::ks_radius(x, y, z, kp.a);
+    even[i] = kp.grid.even ? grt::dev::locate_even(kp.grid, kp.a, x, y, z, r) : grt::dev::kUndecided;
+    stretched[i] = grt::dev::locate_stretched(kp.grid, ax, kp.a, x, y, z, r);
+    exact[i] = grt::dev::locate_exact(kp, ax, x, y, z, r);
+}
+
+__global__ void tetrad_kernel(const double* pos, const double* u, size_t n, double a, double M, uint32_t* out) {
+    const size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
+    if (i >= n) return;
+    const double x = pos[3 * i], y = pos[3 * i + 1], z = pos[3 * i + 2];
+    const double v[4] = {u[4 * i], u[4 * i + 1], u[4 * i + 2], u[4 * i + 3]};
+    const double r = grt::dev::ks_radius(x, y, z, a);
+    grt::dev::MetricAt m;
+    grt::dev::ks_metric_from_r(x, y, z, r, a, M, m);
+    double e[4][4];
+    out[i] = (grt::dev::tetrad_certain(x, y, z, r, a, M, v) ? 1u : 0u) |
+             (grt::dev::build_tetrad(m.g, v, e) ? 2u : 0u) | (grt::dev::build_tetrad<true>(m.g, v, e) ? 4u : 0u);
 }
 
 template <int N>
@@ -194,6 +224,69 @@ int grt_selftest_rhs_bf(const double* states, size_t n, double spin, double M, d
     CK(cudaMemcpy(bf, db, 7 * n * 8, cudaMemcpyDeviceToHost));
     CK(cudaMemcpy(ref, dr, 7 * n * 8, cudaMemcpyDeviceToHost));
     CK(cudaMemcpy(inside, din, n * 4, cudaMemcpyDeviceToHost));
+    return 0;
+}
+
+// Cells of n positions (x, y, z) on the separable grid of the three axes, by
+// locate_even (-2 throughout when the axes are not even), locate_stretched and
+// locate_exact; the two FP32 lookups answer -2 where they do not decide.
+// *is_even receives KGrid::even.
+int grt_selftest_locate(const double* r, int nr, const double* th, int nth, const double* ph, int nph, double spin,
+                        const double* pos, size_t n, int* even, int* stretched, int* exact, int* is_even) {
+    if (n == 0) return 0;
+    const size_t total = static_cast<size_t>(nr) + nth + nph;
+    std::vector<double> host(2 * total);
+    const double* axes[3] = {r, th, ph};
+    const int len[3] = {nr, nth, nph};
+    size_t o = 0;
+    for (int q = 0; q < 3; ++q) {
+        for (int i = 0; i < len[q]; ++i) host[o + i] = axes[q][i];
+        grt::axes::half_spans(axes[q], len[q], q, host.data() + total + o);
+        o += len[q];
+    }
+    Bufs<5> B;
+    double *da, *dp;
+    int *d0, *d1, *d2;
+    CK(B.get(&da, 2 * total));
+    CK(B.get(&dp, 3 * n));
+    CK(B.get(&d0, n));
+    CK(B.get(&d1, n));
+    CK(B.get(&d2, n));
+    CK(cudaMemcpy(da, host.data(), 2 * total * 8, cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(dp, pos, 3 * n * 8, cudaMemcpyHostToDevice));
+    grt::KParams kp{};
+    kp.a = spin;
+    kp.M = 1.0;
+    kp.grid.nr = nr;
+    kp.grid.nth = nth;
+    kp.grid.nph = nph;
+    kp.grid.available = kp.grid.separable = 1;
+    grt::set_axis_lookup(kp.grid, r, th, ph);
+    *is_even = kp.grid.even;
+    const grt::dev::Axes ax{da, da + nr, da + nr + nth, da + total, da + total + nr, da + total + nr + nth};
+    locate_kernel<<<static_cast<unsigned>((n + 127) / 128), 128>>>(kp, ax, dp, n, d0, d1, d2);
+    CK(cudaGetLastError());
+    CK(cudaMemcpy(even, d0, n * 4, cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(stretched, d1, n * 4, cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(exact, d2, n * 4, cudaMemcpyDeviceToHost));
+    return 0;
+}
+
+// out[i]: bit 0 tetrad_certain, bits 1 and 2 build_tetrad's verdict (rolled,
+// unrolled) for four-velocity u[i] at position pos[i].
+int grt_selftest_tetrad(const double* pos, const double* u, size_t n, double spin, double M, uint32_t* out) {
+    if (n == 0) return 0;
+    Bufs<3> B;
+    double *dp, *du;
+    uint32_t* d;
+    CK(B.get(&dp, 3 * n));
+    CK(B.get(&du, 4 * n));
+    CK(B.get(&d, n));
+    CK(cudaMemcpy(dp, pos, 3 * n * 8, cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(du, u, 4 * n * 8, cudaMemcpyHostToDevice));
+    tetrad_kernel<<<static_cast<unsigned>((n + 127) / 128), 128>>>(dp, du, n, spin, M, d);
+    CK(cudaGetLastError());
+    CK(cudaMemcpy(out, d, n * 4, cudaMemcpyDeviceToHost));
     return 0;
 }
 

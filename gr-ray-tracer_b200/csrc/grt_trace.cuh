@@ -109,6 +109,7 @@ struct Lane {
     int fast;             // precision hint of the current call (mixed form)
     int gen_pending;      // backward-leg launch: stopped at first fluid contact, generation left to generate_body
     int need_k1;          // the call's k1 = f(state) is still to be evaluated
+    int scatter_cell;     // disk-mode kernel: cell of the scattering the last call ended with (-1: none)
     double dl_try;
 };
 
@@ -133,6 +134,7 @@ GRT_DEV void load_photon(const KPhotons& P, long long i, Lane& L) {
     L.have_radius = 0;
     L.mid_call = 0;
     L.gen_pending = 0;
+    L.scatter_cell = -1;
     L.zero_all = 0;
 }
 
@@ -422,9 +424,22 @@ struct NoRecord {
     GRT_DEV void zeroed() {}
 };
 
-// Everything after the integration step of one call (integrate_cart_ks.hpp:307-417).
-// phase0 is the phase loaded at the start of the call.  Returns 1 if the photon
-// terminated.
+// Scatters the lane's packet in `cell` at call `step`; false if it did not.
+template <bool RAW>
+GRT_DEV bool scatter_lane(const KParams& kp, Lane& L, int cell, int64_t step) {
+    ScatterState st;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) st.s[c] = L.s[c];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) st.I[q] = L.I[q];
+    if (!scatter_packet<RAW>(kp, &st, cell, L.radius, L.id, step)) return false;
+#pragma unroll
+    for (int c = 4; c < 8; ++c) L.s[c] = st.s[c];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) L.I[q] = st.I[q];
+    return true;
+}
+
 // Packet generation of photon `id` at `step` (integrate_cart_ks.hpp:325-347).
 GRT_DEV bool generate_packet(const KParams& kp, const FluidSample& fs, uint64_t id, int64_t step, int packets,
                              double nu_custom, double& nu, double& E) {
@@ -511,11 +526,15 @@ GRT_DEV int generate_at_contact(const KParams& kp, Lane& L, const FluidSample& f
     return terminated;
 }
 
+// Everything after the integration step of one call (integrate_cart_ks.hpp:307-417).
+// phase0 is the phase loaded at the start of the call.  Returns 1 if the photon
+// terminated.
 // SHARE: the lane also carries the other channels of its group (their
 // frequencies and Stokes vectors in their photon slots); *ch_term counts the
 // channels that terminated on their own in this call.
 // LEG (see trace_body) removes the code the leg never runs: generation from
-// the forward leg, transfer and the camera from the backward leg.
+// the forward leg, transfer and the camera from the backward leg; disk mode
+// (3) leaves a scattering to trace_body (Lane::scatter_cell).
 // radius_hint: the Kerr-Schild radius of L.s when the caller already has it
 // (the mixed form's renormalisation computes it), else negative.  FASTR: the
 // radius through ks_radius_bf (latency-bound instantiations).
@@ -531,8 +550,9 @@ GRT_DEV int post_step(const KParams& kp, const Axes& ax, Lane& L, int phase0, do
     // LEG 3 (disk mode) compiles the image-mode branches out of the step loop
     const bool image_mode = LEG != 3 && kp.image_mode;
     const bool needs = kp.scat_on || kp.abs_on || kp.emis_on || (image_mode && backward);
-    FluidSample fs;
-    const bool sampled = needs && sample_fluid<RAW>(kp, ax, L.s, L.radius, fs);
+    FluidCellCGS fluid;
+    const int cell = needs ? sample_fluid<RAW>(kp, ax, L.s, L.radius, fluid) : -1;
+    const bool sampled = cell >= 0;
     int terminated = 0;
     if (LEG != 2 && image_mode && backward && sampled) {
         if (LEG == 1) {
@@ -540,23 +560,25 @@ GRT_DEV int post_step(const KParams& kp, const Axes& ax, Lane& L, int phase0, do
             // this position again and generates (one call, split)
             L.gen_pending = 1;
         } else {
+            FluidSample fs;
+            full_sample<RAW>(kp, cell, L.s[0], L.s[1], L.s[2], L.s[3], L.radius, &fs);
             terminated = generate_at_contact<SHARE>(kp, L, fs, step, ch_term);
         }
     } else if (LEG != 1 && sampled && !backward) {
         const double I_before = L.I[0];
         double tau0 = 0.0, j0 = 0.0, att = 1.0, scale = 1.0;
         if (kp.abs_on) {
-            double dtau = ComputeOpticalDepthIncrement(fs.fluid, L.freq, taken, im.kappa);
+            double dtau = ComputeOpticalDepthIncrement(fluid, L.freq, taken, im.kappa);
             tau0 = dtau;
-            if (kp.m_abs) dtau = kp.m_abs[fs.cell] * dtau;
+            if (kp.m_abs) dtau = kp.m_abs[cell] * dtau;
             att = exp(-dtau);
 #pragma unroll
             for (int q = 0; q < 4; ++q) L.I[q] *= att;
         }
         if (kp.emis_on) {
-            double dI = ComputeEmissivityIncrement(fs.fluid, L.freq, taken, im.jcoef);
+            double dI = ComputeEmissivityIncrement(fluid, L.freq, taken, im.jcoef);
             j0 = dI;
-            if (kp.m_emis) dI = kp.m_emis[fs.cell] * dI;
+            if (kp.m_emis) dI = kp.m_emis[cell] * dI;
             L.I[0] += dI;
         }
         if (SHARE && (kp.abs_on || kp.emis_on)) {
@@ -567,14 +589,14 @@ GRT_DEV int post_step(const KParams& kp, const Axes& ax, Lane& L, int phase0, do
                 const double f_c = kp.ph.frequency[sc];
                 double Ic[4] = {kp.ph.I[sc], kp.ph.Q[sc], kp.ph.U[sc], kp.ph.V[sc]};
                 if (kp.abs_on) {
-                    double dtau = ComputeOpticalDepthIncrement(fs.fluid, f_c, taken, ic.kappa);
-                    if (kp.m_abs) dtau = kp.m_abs[fs.cell] * dtau;
+                    double dtau = ComputeOpticalDepthIncrement(fluid, f_c, taken, ic.kappa);
+                    if (kp.m_abs) dtau = kp.m_abs[cell] * dtau;
                     const double att_c = exp(-dtau);
                     for (int q = 0; q < 4; ++q) Ic[q] *= att_c;
                 }
                 if (kp.emis_on) {
-                    double dI = ComputeEmissivityIncrement(fs.fluid, f_c, taken, ic.jcoef);
-                    if (kp.m_emis) dI = kp.m_emis[fs.cell] * dI;
+                    double dI = ComputeEmissivityIncrement(fluid, f_c, taken, ic.jcoef);
+                    if (kp.m_emis) dI = kp.m_emis[cell] * dI;
                     Ic[0] += dI;
                 }
                 kp.ph.I[sc] = Ic[0];
@@ -585,22 +607,12 @@ GRT_DEV int post_step(const KParams& kp, const Axes& ax, Lane& L, int phase0, do
         }
         if (kp.scat_on) {
             Philox rng(kp.seed, L.id, static_cast<uint32_t>(step));
-            if (scatter_drawn(fabs(L.dl), kp.length_scale, fs, rng)) {
-                ScatterState st;
-#pragma unroll
-                for (int c = 0; c < 8; ++c) st.s[c] = L.s[c];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) st.I[q] = L.I[q];
-                if (scatter_packet(&st, kp.albedo, fs, kp.a, kp.M, &rng)) {
-#pragma unroll
-                    for (int c = 4; c < 8; ++c) L.s[c] = st.s[c];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) L.I[q] = st.I[q];
-                    scale = kp.albedo;
-                }
+            if (scatter_drawn(fabs(L.dl), kp.length_scale, fluid, rng)) {
+                if (LEG == 3) L.scatter_cell = cell;  // trace_body scatters it
+                else if (scatter_lane<RAW>(kp, L, cell, step)) scale = kp.albedo;
             }
         }
-        rec.rt_step(fs.cell, tau0, j0, I_before, att, scale);
+        rec.rt_step(cell, tau0, j0, I_before, att, scale);
     }
     if (LEG != 1 && image_mode && phase0 == 2) {  // ImageForward
         double u = 0.0, v = 0.0;
@@ -672,6 +684,7 @@ GRT_DEV void trace_body(const KParams& kp, const Axes& ax, const KStore& kk) {
     const unsigned lt_mask = (1u << lane) - 1u;
     Lane L;
     L.idx = -1;
+    L.scatter_cell = -1;
     LaneCounters cnt = {0, 0, 0, 0, 0};
     bool exhausted = false;
     bool first_claim = true;
@@ -772,6 +785,23 @@ GRT_DEV void trace_body(const KParams& kp, const Axes& ax, const KStore& kk) {
             timed_out = true;
             break;
         }
+        if (LEG == 3) {
+            // A packet that scatters waits for company: its new direction takes
+            // a tetrad, 1,000 FP64 instructions or so that a warp issues whole
+            // for one lane as for many.  Once a quarter of the live lanes wait
+            // (so that a lone lane never does) they scatter together.  One by
+            // one, some lane of nearly every warp iteration held the other 31:
+            // 2.07e6 packets 63.1 ms, with a scattering turned off 21.9.
+            const unsigned waiting = __ballot_sync(kFull, L.idx >= 0 && L.scatter_cell >= 0);
+            if (4 * __popc(waiting) >= __popc(active)) {
+                if (L.idx >= 0 && L.scatter_cell >= 0) {
+                    scatter_lane<RAW>(kp, L, L.scatter_cell, kp.step0 + L.calls - 1);
+                    L.scatter_cell = -1;
+                }
+                __syncwarp();
+            }
+            if (L.idx >= 0 && L.scatter_cell >= 0) continue;
+        }
         if (L.idx < 0) continue;
 
         // ---- one unit of work for this lane ----
@@ -868,6 +898,7 @@ GRT_DEV void trace_body(const KParams& kp, const Axes& ax, const KStore& kk) {
     if (timed_out) {
         // Leave every photon consistent: write back what this lane holds.
         if (L.idx >= 0) {
+            if (LEG == 3 && L.scatter_cell >= 0) scatter_lane<RAW>(kp, L, L.scatter_cell, kp.step0 + L.calls - 1);
             store_all<SHARE, LEG == 1>(kp, L, 0, tdisp, pdisp, have_disp);
             store_carry<SHARE, LEG>(kp, L);
         }
@@ -934,7 +965,8 @@ GRT_DEV void generate_body(const KParams& kp, const Axes& ax) {
         L.have_radius = 1;
         FluidSample fs;
         int ch_term = 0, term = 0;
-        if (sample_fluid<false>(kp, ax, L.s, L.radius, fs))
+        const int cell = locate_fluid(kp, ax, L.s[1], L.s[2], L.s[3], L.radius);
+        if (cell >= 0 && full_sample<false>(kp, cell, L.s[0], L.s[1], L.s[2], L.s[3], L.radius, &fs))
             term = generate_at_contact<SHARE>(kp, L, fs, kp.step0 + L.calls - 1, &ch_term);
         if (term || ch_term) {
             const unsigned long long ts = static_cast<unsigned long long>(kp.step0 + L.calls);
