@@ -66,6 +66,15 @@ __device__ __forceinline__ bool div_zero_or_within(double v) {
     return e == 0u ? (v == 0.0) : (e - static_cast<unsigned>(1023 + LO)) <= static_cast<unsigned>(HI - LO);
 }
 
+// The smallest of m and the high word of |v|, an exact zero counting as large:
+// a chain over several values ends at or above (1023 + lo) << 20, less one,
+// when each is a zero or at least 2^lo (to within one part in 2^20).
+__device__ __forceinline__ unsigned div_min_nonzero(unsigned m, double v) {
+    const unsigned hi = static_cast<unsigned>(__double2hiint(v)) & 0x7FFFFFFFu;
+    const unsigned lo = static_cast<unsigned>(__double2loint(v));
+    return min(m, hi + min(lo, 1u) - 1u);  // zero wraps; a subnormal stays small
+}
+
 // 2^lo <= |v| < 2^(hi+1), v finite and normal.
 template <int LO, int HI>
 __device__ __forceinline__ bool div_within(double v) {

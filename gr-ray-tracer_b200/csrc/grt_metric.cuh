@@ -132,22 +132,26 @@ GRT_DEV Rhs7 ks_rhs(double x, double y, double z, double pt, double px, double p
 // its denominator (six of them: S, 2r, B, r, D, D^2; five reciprocal
 // evaluations, since RN(1/(2r)) = RN(1/r) / 2) by div_by, which rounds like an
 // IEEE division while no value under- or overflows.  That holds in
-// the box this checks first: x, y, z each an exact zero or of magnitude in
+// the box this checks: x, y, z each an exact zero or of magnitude in
 // [2^-20, 2^20], r in [2^-24, 2^20] and S in [2^-60, 2^42], with a spin of
 // magnitude 0 or in [2^-20, 2] and a mass in [2^-20, 2^20] (checked on the
 // host: rcp_ok).  Inside it every numerator, quotient and denominator stays
 // in [2^-900, 2^900]: products of at most eight factors of at least 2^-60,
 // differences of such products (zero, or at least 2^-52 of the smaller),
-// divided by at most r^8 <= 2^160.  Outside it `ok` is false and the caller
-// evaluates ks_rhs.  The expression tree is ks_rhs's, so the result equals
-// ks_rhs bit for bit.
+// divided by at most r^8 <= 2^160.  Outside it, and where a denominator's low
+// word is all ones (once in 2^32: it covers the one significand that
+// rcp_rn_core does not round), `ok` is false and the caller evaluates ks_rhs.
+// The expression tree is ks_rhs's, so the result equals ks_rhs bit for bit.
+// The check comes last: nothing here traps, and without a branch in the middle
+// the right-hand side is one block for the compiler to schedule.  The upper
+// bounds of x, y and z are those of r (|z| <= r, x^2 + y^2 <= r^2 + a^2).
 // BF selects the branch-free reciprocal and square root of grt_rn.cuh (equal
 // to __drcp_rn and sqrt on every argument that reaches them here: the square
-// roots' results are checked against the box before use, and every
-// reciprocal's argument lies in [2^-192, 2^164]); without it, CUDA's.
+// roots' results are checked against the box, and every reciprocal's argument
+// lies in [2^-192, 2^164]); without it, CUDA's.
 template <bool BF>
 GRT_DEV double rhs_recip(double b) {
-    if constexpr (BF) return rcp_rn_box(b);
+    if constexpr (BF) return rcp_rn_core(b);
     else return div_recip(b);
 }
 
@@ -156,6 +160,8 @@ GRT_DEV double rhs_sqrt(double v) {
     if constexpr (BF) return sqrt_rn_box(v);
     else return sqrt(v);
 }
+
+GRT_DEV unsigned low_word(double v) { return static_cast<unsigned>(__double2loint(v)); }
 
 template <bool BF = false>
 GRT_DEV Rhs7 ks_rhs_rcp(double x, double y, double z, double pt, double px, double py, double pz,
@@ -167,10 +173,7 @@ GRT_DEV Rhs7 ks_rhs_rcp(double x, double y, double z, double pt, double px, doub
     // measured 3% faster on a lane-per-SM workload than one rolled site.
     const double S = rhs_sqrt<BF>(A * A + 4.0 * ((a * z) * (a * z)));
     const double r = rhs_sqrt<BF>(0.5 * (A + S));
-    ok = div_zero_or_within<-20, 19>(x) && div_zero_or_within<-20, 19>(y) && div_zero_or_within<-20, 19>(z) &&
-         div_within<-24, 19>(r) && div_within<-60, 41>(S);
-    Rhs7 o{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    if (!ok) return o;
+    Rhs7 o;
     const double yS = rhs_recip<BF>(S);
     const double opas = 1.0 + div_by(A, S, yS);
     const double two_r = 2.0 * r;
@@ -213,6 +216,9 @@ GRT_DEV Rhs7 ks_rhs_rcp(double x, double y, double z, double pt, double px, doub
     const double dH0 = div_by(M * (three_r2 * dr0 * D - r3 * dD0), DD, yDD);
     const double dH1 = div_by(M * (three_r2 * dr1 * D - r3 * dD1), DD, yDD);
     const double dH2 = div_by(M * (three_r2 * dr2 * D - r3 * dD2), DD, yDD);
+    const unsigned small = div_min_nonzero(div_min_nonzero(div_min_nonzero(~0u, x), y), z);
+    const unsigned ones = max(max(max(low_word(S), low_word(r)), max(low_word(B), low_word(D))), low_word(DD));
+    ok = small >= ((1023u - 20u) << 20) - 1u && div_within<-24, 19>(r) && div_within<-60, 41>(S) && ones != ~0u;
     const double ldp = ((-pt + l1 * px) + l2 * py) + l3 * pz;
     const double twoH = 2.0 * H;
     o.t = -pt - (-twoH) * ldp;

@@ -59,12 +59,17 @@ __device__ __forceinline__ double rsqrt_seed(double v) {
     return y;
 }
 
-__device__ __forceinline__ double rcp_rn_box(double b) {
+// RN(1/b) unless b's significand is all ones.
+__device__ __forceinline__ double rcp_rn_core(double b) {
     double y = rcp_seed(b);
     double e = fma(-b, y, 1.0);
     y = fma(y, fma(e, e, e), y);
     e = fma(-b, y, 1.0);
-    y = fma(y, e, y);
+    return fma(y, e, y);
+}
+
+__device__ __forceinline__ double rcp_rn_box(double b) {
+    const double y = rcp_rn_core(b);
     // all-ones significand: RN(1/b) = sign(b) 2^(-E-1) (1 + 2^-52); with b's
     // biased exponent eb = E + 1023 that is biased exponent 2045 - eb
     const unsigned hi = static_cast<unsigned>(__double2hiint(b));
