@@ -237,13 +237,11 @@ grt_status cuda_fail(grt_ctx* c, cudaError_t e, const char* what) {
         if (e_ != cudaSuccess) return cuda_fail(ctx, e_, what); \
     } while (0)
 
-// fluid_frame.hpp:28-48 on the host (glibc sin/cos, exactly the reference's
-// arithmetic), then the [units] scale, as sample_scattering_fluid applies it
+// fluid_frame.hpp:28-48 on the host (sines and cosines of the cell's angles by
+// glibc, exactly the reference's arithmetic), then the [units] scale, as sample_scattering_fluid applies it
 // per step (scattering.hpp:223-241).
-void spherical_to_cartesian_vec(double r, double th, double ph, double spin, const double s[4], double scale,
-                                double c[4]) {
-    const double st = std::sin(th), ct = std::cos(th);
-    const double sp = std::sin(ph), cp = std::cos(ph);
+void spherical_to_cartesian_vec(double r, double st, double ct, double sp, double cp, double spin, const double s[4],
+                                double scale, double c[4]) {
     const double radial_x = cp * st, radial_y = sp * st, radial_z = ct;
     const double theta_x = (r * cp - spin * sp) * ct;
     const double theta_y = (r * sp + spin * cp) * ct;
@@ -551,8 +549,8 @@ grt_status grt_upload_grid(grt_ctx* c, size_t nr, size_t nth, size_t nph, const 
         pos[3 * q + 1] = (r[q] * sp + c->p.spin * cp) * st;
         pos[3 * q + 2] = r[q] * ct;
         double u[4], b[4];
-        spherical_to_cartesian_vec(r[q], th[q], ph[q], c->p.spin, vel4 + 4 * q, c->p.four_velocity_cm_s_per_code, u);
-        spherical_to_cartesian_vec(r[q], th[q], ph[q], c->p.spin, mag4 + 4 * q, c->p.magnetic_gauss_per_code, b);
+        spherical_to_cartesian_vec(r[q], st, ct, sp, cp, c->p.spin, vel4 + 4 * q, c->p.four_velocity_cm_s_per_code, u);
+        spherical_to_cartesian_vec(r[q], st, ct, sp, cp, c->p.spin, mag4 + 4 * q, c->p.magnetic_gauss_per_code, b);
         uv[2 * q] = make_double2(u[0], u[1]);
         uv[2 * q + 1] = make_double2(u[2], u[3]);
         bv[2 * q] = make_double2(b[0], b[1]);

@@ -255,8 +255,8 @@ static __constant__ double kFehlbergA[5][5] = {
 constexpr int kTraceThreads = 128;
 
 // Per-thread slots in shared memory: the stage derivatives k1..k5 (slots
-// 0..4; k6 replaces k2 in slot 1 once the last stage input is formed) and the
-// state (slot 5) for the error norm.  [6][7][kTraceThreads] doubles,
+// 0..4) and, for the rolled error norm, k6 in place of k2 in slot 1 and the
+// state in slot 5.  [6][7][kTraceThreads] doubles,
 // thread-contiguous so a warp's accesses are conflict-free; base already
 // points at this thread's column, so a slot is a constant offset from it.
 // k1 stays there across the retries of one call.
@@ -270,6 +270,21 @@ struct KStore {
 // (grt_pow_quarter.cuh); out of line to keep the step loop small.
 static __device__ __noinline__ double controller_root(double x) { return pow_quarter(x); }
 
+// max(|u|, |v|) for numbers; a NaN gives a NaN (non-negative doubles order as
+// their bit patterns).
+GRT_DEV double larger_magnitude(double u, double v) {
+    return __longlong_as_double(max(__double_as_longlong(fabs(u)), __double_as_longlong(fabs(v))));
+}
+
+// (n, sc) becomes the pair of larger exact ratio of (n, sc) and (m, sd).
+GRT_DEV void larger_ratio(double& n, double& sc, double m, double sd) {
+    const double p = m * sc, q = n * sd;
+    if (p > q || (p == q && fma(m, sc, -p) > fma(n, sd, -q))) {
+        n = m;
+        sc = sd;
+    }
+}
+
 // One Fehlberg attempt (integrate_cart_ks.hpp:159-227), preceded by the
 // call's k1 = f(state) when need_k1 (integrate_cart_ks.hpp:274-275); returns 1
 // if accepted (s advanced), 0 if rejected; *dl receives the next proposed step
@@ -277,17 +292,29 @@ static __device__ __noinline__ double controller_root(double x) { return pow_qua
 // loop -- a lane that needs k1 runs it one iteration ahead of the others, so
 // the warp stays converged on the same code -- and the derivatives live in
 // shared memory (KStore), which keeps registers for the right-hand side.
-// The stage sums and the error norm are rolled loops too, the norm with a
-// single division site: every inline IEEE division brings its slow path into
-// the step loop's instruction stream, and with seven of them unrolled the
-// loop missed the instruction cache far more (the unrolled form was 11-22%
-// slower on C2 and C3).  Each stage input is summed over j = 1..t-1 left to
-// right, the reference's association; for the first stage, dt*(a21 k1)
-// equals the reference's (dt*a21)*k1 because a21 = 1/4 is a power of two.
-template <class RHS>
+// Each stage input is summed over j = 1..t-1 left to right, the reference's
+// association; for the first stage, dt*(a21 k1) equals the reference's
+// (dt*a21)*k1 because a21 = 1/4 is a power of two.
+//
+// The error norm is max_c RN(n_c / sc_c).  Rounding is monotone, so it equals
+// RN(n_m / sc_m) for the component m of largest exact ratio, found by
+// comparing exact cross products n_c sc_m against n_m sc_c (the product and
+// its fma residual): one division instead of seven.  That needs every n_c,
+// sc_c inside [2^-400, 2^400] (or n_c = 0), so that no product under- or
+// overflows and no x4, x5 is infinite or NaN; otherwise the ratios are formed
+// one by one.
+// WIDE: the norm's components as straight-line code in registers.  Rolled, its
+// seven chains run one after another through shared memory, a third of a lone
+// warp's attempt.  Trace ms rolled / wide: 256 rays 0.468 / 0.426, adjoint
+// forward of 16,384 rays 1.80 / 1.62, 65,536 rays 1.010 / 0.986, 4.76e6 rays
+// 33.97 / 33.49.  The disk-mode loop, with the sample, transfer and scattering
+// of every step in it, outgrows the instruction cache: 2.07e6 packets 46.1 /
+// 49.1 at 4 blocks/SM, so it stays rolled.
+template <class RHS, bool WIDE>
 GRT_DEV int rk45_attempt(const KParams& kp, double s[8], double* dl, int need_k1, int fast, const KStore& kk) {
     const double dt = *dl;
     double t[8];
+    V7 k;
     t[4] = s[4];
 #pragma unroll 1
     for (int st = need_k1 ? -1 : 0; st < 5; ++st) {
@@ -308,58 +335,77 @@ GRT_DEV int rk45_attempt(const KParams& kp, double s[8], double* dl, int need_k1
 #pragma unroll
             for (int c = 0; c < 7; ++c) t[sidx(c)] = s[sidx(c)] + dt * acc[c];
         }
-        const V7 k = RHS::eval(t, kp, fast);
-        // k2..k5 to slots 1..4; k6 replaces k2 in slot 1 (no later use)
-        const int slot = st < 4 ? st + 1 : 1;
+        k = RHS::eval(t, kp, fast);
+        // k1..k5 to slots 0..4; rolled, k6 replaces k2 in slot 1 (no later use)
+        if (!WIDE || st < 4) {
+            const int slot = st < 4 ? st + 1 : 1;
 #pragma unroll
-        for (int c = 0; c < 7; ++c) kk.at(slot, c) = k.v[c];
+            for (int c = 0; c < 7; ++c) kk.at(slot, c) = k.v[c];
+        }
     }
-    // The state goes to slot 5 so that the error norm runs as a loop over the
-    // components (one division site); x5 replaces it there.
-#pragma unroll
-    for (int c = 0; c < 7; ++c) kk.at(5, c) = s[sidx(c)];
-    double err = 0.0;
-    bool finite = isfinite(s[4]);
-    // The norm is max_c RN(n_c / sc_c).  Rounding is monotone, so it equals
-    // RN(n_m / sc_m) for the component m of largest exact ratio, found by
-    // comparing exact cross products n_c sc_m against n_m sc_c (the product
-    // and its fma residual).  One division then replaces seven serial ones.
-    // That needs every x4, x5 finite and n_c, sc_c inside [2^-400, 2^400]
-    // (or n_c = 0), so that no product under- or overflows; otherwise the
-    // ratios are formed one by one as before.  n_c and sc_c go to slots 2
-    // and 3 (k3, k4: not read again in this attempt).
+    double x5[7], nm, sm;
     bool boxed = true;
-#pragma unroll 1
-    for (int c = 0; c < 7; ++c) {
-        const double si = kk.at(5, c);
-        const double k1 = kk.at(0, c), k3 = kk.at(2, c), k4 = kk.at(3, c), k5 = kk.at(4, c), k6 = kk.at(1, c);
-        const double x4 = si + dt * (b41 * k1 + b43 * k3 + b44 * k4 + b45 * k5);
-        const double x5 = si + dt * (b51 * k1 + b53 * k3 + b54 * k4 + b55 * k5 + b56 * k6);
-        const double sc = kp.atol + kp.rtol * fmax(fabs(x5), fabs(x4));
-        const double n = fabs(x5 - x4);
-        boxed = boxed && isfinite(x4) && isfinite(x5) && div_within<-400, 399>(sc) &&
-                div_zero_or_within<-400, 399>(n);
-        kk.at(5, c) = x5;
-        kk.at(2, c) = n;
-        kk.at(3, c) = sc;
-    }
-    if (boxed) {
-        double nm = kk.at(2, 0), sm = kk.at(3, 0);
-#pragma unroll 1
-        for (int c = 1; c < 7; ++c) {
-            const double n = kk.at(2, c), sc = kk.at(3, c);
-            const double p = n * sm, q = nm * sc;
-            if (p > q || (p == q && fma(n, sm, -p) > fma(nm, sc, -q))) {
-                nm = n;
-                sm = sc;
+    if constexpr (WIDE) {
+        double n[7], sc[7];
+#pragma unroll
+        for (int c = 0; c < 7; ++c) {
+            const double si = s[sidx(c)];
+            const double k1 = kk.at(0, c), k3 = kk.at(2, c), k4 = kk.at(3, c), k5 = kk.at(4, c), k6 = k.v[c];
+            const double x4 = si + dt * (b41 * k1 + b43 * k3 + b44 * k4 + b45 * k5);
+            x5[c] = si + dt * (b51 * k1 + b53 * k3 + b54 * k4 + b55 * k5 + b56 * k6);
+            sc[c] = kp.atol + kp.rtol * larger_magnitude(x5[c], x4);
+            n[c] = fabs(x5[c] - x4);
+            boxed = boxed && div_within<-400, 399>(sc[c]) && div_zero_or_within<-400, 399>(n[c]);
+        }
+        if (!boxed) {  // for the loop of divisions below; k4, k6 are read before they go
+#pragma unroll
+            for (int c = 0; c < 7; ++c) {
+                const double k1 = kk.at(0, c), k3 = kk.at(2, c), k4 = kk.at(3, c), k5 = kk.at(4, c);
+                const double x4 = s[sidx(c)] + dt * (b41 * k1 + b43 * k3 + b44 * k4 + b45 * k5);
+                kk.at(1, c) = x5[c];
+                kk.at(2, c) = n[c];
+                kk.at(3, c) = kp.atol + kp.rtol * fmax(fabs(x5[c]), fabs(x4));
             }
         }
+        larger_ratio(n[0], sc[0], n[1], sc[1]);
+        larger_ratio(n[2], sc[2], n[3], sc[3]);
+        larger_ratio(n[4], sc[4], n[5], sc[5]);
+        larger_ratio(n[0], sc[0], n[2], sc[2]);
+        larger_ratio(n[4], sc[4], n[6], sc[6]);
+        larger_ratio(n[0], sc[0], n[4], sc[4]);
+        nm = n[0];
+        sm = sc[0];
+    } else {
+        // the state goes to slot 5 so that the components run as a loop; x5
+        // ends in slot 1 (k2 and k6: not read again), n and sc in slots 2 and 3
+#pragma unroll
+        for (int c = 0; c < 7; ++c) kk.at(5, c) = s[sidx(c)];
+        nm = 0.0;
+        sm = 1.0;
+#pragma unroll 1
+        for (int c = 0; c < 7; ++c) {
+            const double si = kk.at(5, c);
+            const double k1 = kk.at(0, c), k3 = kk.at(2, c), k4 = kk.at(3, c), k5 = kk.at(4, c), k6 = kk.at(1, c);
+            const double x4 = si + dt * (b41 * k1 + b43 * k3 + b44 * k4 + b45 * k5);
+            const double x = si + dt * (b51 * k1 + b53 * k3 + b54 * k4 + b55 * k5 + b56 * k6);
+            const double sc = kp.atol + kp.rtol * fmax(fabs(x), fabs(x4));
+            const double n = fabs(x - x4);
+            boxed = boxed && div_within<-400, 399>(sc) && div_zero_or_within<-400, 399>(n);
+            kk.at(1, c) = x;
+            kk.at(2, c) = n;
+            kk.at(3, c) = sc;
+            larger_ratio(nm, sm, n, sc);
+        }
+    }
+    double err = 0.0;
+    bool finite = isfinite(s[4]);
+    if (boxed) {
         err = div_by(nm, sm, div_recip(sm));
     } else {
 #pragma unroll 1
         for (int c = 0; c < 7; ++c) {
             const double ratio = kk.at(2, c) / kk.at(3, c);
-            if (!isfinite(kk.at(5, c)) || !isfinite(ratio)) finite = false;
+            if (!isfinite(kk.at(1, c)) || !isfinite(ratio)) finite = false;
             err = fmax(err, ratio);
         }
     }
@@ -367,23 +413,18 @@ GRT_DEV int rk45_attempt(const KParams& kp, double s[8], double* dl, int need_k1
         *dl = dt * kp.min_scale;
         return 0;
     }
-    if (err == 0.0) {
-        *dl = dt * kp.max_scale;
-#pragma unroll
-        for (int c = 0; c < 7; ++c) s[sidx(c)] = kk.at(5, c);
-        return 1;
+    double scale = kp.max_scale;
+    if (err != 0.0) {
+        // 1/err rounded to nearest, as the division 1.0 / err rounds it (err is
+        // finite and positive here), without a second division site
+        scale = kp.safety * controller_root(div_recip(err));
+        scale = fmin(kp.max_scale, fmax(kp.min_scale, scale));
     }
-    // 1/err rounded to nearest, as the division 1.0 / err rounds it (err is
-    // finite and positive here), without a second division site
-    double scale = kp.safety * controller_root(div_recip(err));
-    scale = fmin(kp.max_scale, fmax(kp.min_scale, scale));
     *dl = dt * scale;
-    if (err <= 1.0) {
+    if (!(err <= 1.0)) return 0;
 #pragma unroll
-        for (int c = 0; c < 7; ++c) s[sidx(c)] = kk.at(5, c);
-        return 1;
-    }
-    return 0;
+    for (int c = 0; c < 7; ++c) s[sidx(c)] = WIDE ? x5[c] : kk.at(1, c);
+    return 1;
 }
 
 struct LaneCounters {
@@ -856,7 +897,7 @@ GRT_DEV void trace_body(const KParams& kp, const Axes& ax, const KStore& kk) {
             const double taken = L.dl_try;
             // the backward leg never uses the FP32 right-hand side (a literal
             // 0 lets the compiler drop it from the backward kernel)
-            const int ok = rk45_attempt<RHS>(kp, L.s, &L.dl_try, L.need_k1, LEG == 1 ? 0 : L.fast, kk);
+            const int ok = rk45_attempt<RHS, LEG != 3>(kp, L.s, &L.dl_try, L.need_k1, LEG == 1 ? 0 : L.fast, kk);
             L.need_k1 = 0;
             ++L.attempts;
             if (ok) {
