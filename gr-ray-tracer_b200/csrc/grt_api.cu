@@ -1091,13 +1091,21 @@ grt_status prepare_trace_buffers(grt_ctx* c, unsigned long long queue) {
 // first fluid contact, and, with the queue head reset, the forward-leg launch
 // over the same queue.
 // Resident trace blocks per SM: the launch shape's, or with 0 (automatic)
-// the fewest of 2, 3, 4 that keep every geodesic of the queue resident at
-// once -- fewer blocks give each thread more registers (255, 170, 128) and
-// spill less, and a workload that fits needs no more lanes.
+// in image mode the fewest of 2, 3, 4 that keep every geodesic of the queue
+// resident at once -- fewer blocks give each thread more registers (255, 170,
+// 128) and spill less, and a workload that fits needs no more lanes.  Disk
+// packets live from a few calls to hundreds and a warp keeps its lanes filled
+// from the queue, so residency does not matter; the longest packets' latency
+// and the instruction cache do.  Trace ms at 2 / 3 / 4 blocks: 1.3e4 packets
+// 2.85 / 3.23 / 4.16, 1.1e5 4.70 / 5.39 / 6.81, 3.4e5 9.08 / 9.29 / 11.0, 5.7e5
+// 14.2 / 13.8 / 15.9, 2.07e6 45.2 / 42.4 / 46.2: 3 above eight packets for
+// every lane of 2 blocks, 2 below.
 int trace_blocks_per_sm(const grt_ctx* c, unsigned long long queue) {
     if (c->lc.blocks_per_sm) return c->lc.blocks_per_sm;
+    const unsigned long long lanes = static_cast<unsigned long long>(c->sm_count) * 128;
+    if (c->p.mode == GRT_MODE_DISK) return queue <= 8 * 2 * lanes ? 2 : 3;
     for (int b = 2; b < 4; ++b)
-        if (static_cast<unsigned long long>(c->sm_count) * b * 128 >= queue) return b;
+        if (lanes * b >= queue) return b;
     return 4;
 }
 
