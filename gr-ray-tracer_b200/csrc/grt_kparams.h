@@ -122,6 +122,16 @@ struct KParams {
     int64_t budget;            // calls each live photon may take in this launch
     unsigned long long max_iterations;  // per-warp loop limit (GRT_ETIMEOUT)
     KCounters* counters;
+    // Chunked step loop (termination_percent < 1): chunks are enqueued several
+    // at a time, chunk i with its own counters; its blocks return at once when
+    // the counters of the n_prior chunks before it (complete: stream order)
+    // show the run stopped -- the terminated fraction reached, or a time-out.
+    const KCounters* prior;
+    int n_prior;
+    int pad_prior;
+    unsigned long long prior_terminated;  // photons terminated before the first of them
+    unsigned long long total;             // photons the fraction divides by
+    double stop_fraction;
     // two-launch image mode (trace_body LEG 1 then 2): calls each photon took
     // in the backward-leg launch, by queue index, zeroed before it
     long long* calls_carry;

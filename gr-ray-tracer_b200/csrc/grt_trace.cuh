@@ -1037,6 +1037,19 @@ GRT_DEV void generate_body(const KParams& kp, const Axes& ax) {
     }
 }
 
+// Whether the step loop has stopped before this launch's chunk (KParams::prior):
+// the reference's test after each earlier output step, in its arithmetic
+// (integrate_cart_ks.hpp:496-526).
+GRT_DEV bool run_stopped(const KParams& kp) {
+    unsigned long long terminated = kp.prior_terminated;
+    for (int c = 0; c < kp.n_prior; ++c) {
+        if (kp.prior[c].timed_out) return true;
+        terminated += kp.prior[c].terminated;
+        if (static_cast<double>(terminated) / static_cast<double>(kp.total) >= kp.stop_fraction) return true;
+    }
+    return false;
+}
+
 // Shared-memory layout of a trace block: [stage slots (RK45)] [axes and
 // half-spans of a separable grid].  Returns the staged pointers.
 GRT_DEV void stage_grid(const KParams& kp, double* smem, int integrator, Axes& ax, KStore& kk) {

@@ -31,6 +31,7 @@ namespace grt {
 template <int INTEGRATOR, int MINB, bool SHARE, int LEG>
 __global__ void __launch_bounds__(128, MINB) GRT_TRACE_KERNEL(const __grid_constant__ KParams kp) {
     extern __shared__ double smem[];
+    if (kp.n_prior && dev::run_stopped(kp)) return;
     dev::Axes ax;
     dev::KStore kk;
     dev::stage_grid(kp, smem, INTEGRATOR, ax, kk);
@@ -84,6 +85,7 @@ cudaError_t GRT_LAUNCHER(const KParams& kp, int integrator, int blocks_per_sm, i
 template <bool SHARE>
 __global__ void __launch_bounds__(128) generate_pending(const __grid_constant__ KParams kp) {
     extern __shared__ double smem[];
+    if (kp.n_prior && dev::run_stopped(kp)) return;
     dev::Axes ax;
     dev::KStore kk;
     dev::stage_grid(kp, smem, 0, ax, kk);
