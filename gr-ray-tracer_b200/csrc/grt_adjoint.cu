@@ -17,9 +17,15 @@
 // state where its radiative transfer starts -- right after the emission call
 // of an image-backward ray, at the start for forward and disk photons -- and
 // every K calls after that.
-// adj_reverse walks each arrived ray's checkpoints from the last to the first:
-// it recomputes the K calls of a segment from its checkpoint, recording the
-// RT updates on a per-ray tape, then sweeps the tape backwards.
+// It also records the transfer updates of the first AdjointArgs::full_cap
+// sampled steps of a ray (rays of a 128 x 128 image take about 25; 48 bytes
+// each, so memory is no reason to compute them twice on this card).
+// adj_sweep sweeps the recorded rays backwards; nothing is traced again.
+// adj_reverse takes the rays that sampled more: it walks an arrived ray's
+// checkpoints from the last to the first, recomputes the K calls of a segment
+// from its checkpoint, recording the RT updates on a per-ray tape, then sweeps
+// the tape backwards.  With a record for every ray the reverse pass of 16,384
+// rays takes GRT_SWEEP instead of a second trace.
 #include "grt_launch.h"
 #include "grt_trace.cuh"
 
@@ -92,6 +98,41 @@ GRT_DEV int run_call(const KParams& kp, const Axes& ax, const KStore& kk, Lane& 
     return 1;  // integrate_cart_ks.hpp:294-297: give up, phase and state unchanged
 }
 
+// The forward pass's record (AdjointArgs::full) of ray i.
+struct FullRecord {
+    double* full;
+    long long n, i;
+    int* count;
+    int cap;
+    GRT_DEV void rt_step(int cell, double tau0, double j0, double I_before, double att, double scale) const {
+        const int t = *count;
+        if (t < cap) {
+            const double v[kTapeDoubles] = {static_cast<double>(cell), tau0, j0, I_before, att, scale};
+#pragma unroll
+            for (int f = 0; f < kTapeDoubles; ++f) full[(static_cast<long long>(t) * kTapeDoubles + f) * n + i] = v[f];
+        }
+        *count = t + 1;
+    }
+    // the arriving Stokes vector was zeroed: it depends on nothing
+    GRT_DEV void zeroed() const { *count = 0; }
+};
+
+// dL/dI of an arrived ray's pixel.
+GRT_DEV double pixel_adjoint(const KParams& kp, const AdjointArgs& aa, long long i) {
+    const unsigned long long px = observation_bin(kp.ph.theta_disp[i], -0.5 * aa.W, 0.5 * aa.W, aa.nx);
+    const unsigned long long py = observation_bin(kp.ph.phi_disp[i], -0.5 * aa.H, 0.5 * aa.H, aa.ny);
+    return aa.dL_dI[py * aa.nx + px];
+}
+
+// One transfer update swept backwards: adds its gradients, returns dL/dI before it.
+GRT_DEV double sweep_step(const KParams& kp, const AdjointArgs& aa, double lam, int cell, double tau0, double j0,
+                          double I_before, double att, double scale) {
+    const double lp = lam * scale;
+    if (kp.emis_on) atomicAdd(aa.g_emis + cell, lp * j0);
+    if (kp.abs_on) atomicAdd(aa.g_abs + cell, lp * I_before * att * (-tau0));
+    return lp * att;
+}
+
 struct TapeRecord {
     double* tape;  // this thread's K entries
     int* count;
@@ -127,13 +168,15 @@ __global__ void __launch_bounds__(128, 2) adj_forward(const __grid_constant__ KP
          i < static_cast<long long>(kp.n); i += stride) {
         aa.nckpt[i] = 0;
         aa.call0[i] = -1;
+        aa.nfull[i] = 0;
         if (kp.ph.terminate[i]) continue;
         dev::Lane L;
         dev::load_photon(kp.ph, i, L);
         L.idx = i;
         L.img = dev::image_of_photon(kp, i);
         double tdisp = 0.0, pdisp = 0.0;
-        int have_disp = 0, terminated = 0, nck = 0;
+        int have_disp = 0, terminated = 0, nck = 0, count = 0;
+        const dev::FullRecord rec{aa.full, static_cast<long long>(kp.n), i, &count, aa.full_cap};
         // radiative transfer starts after the emission call (image backward
         // rays) or at once (forward and disk photons)
         long long c0 = L.phase == 1 ? -1 : 0;
@@ -147,15 +190,36 @@ __global__ void __launch_bounds__(128, 2) adj_forward(const __grid_constant__ KP
                 }
             }
             const int phase_before = L.phase;
-            terminated = dev::run_call<INTEGRATOR>(kp, ax, kk, L, tdisp, pdisp, have_disp, dev::NoRecord());
+            terminated = dev::run_call<INTEGRATOR>(kp, ax, kk, L, tdisp, pdisp, have_disp, rec);
             if (terminated) break;
             if (c0 < 0 && phase_before == 1 && L.phase == 2) c0 = L.calls;  // emitted in this call
         }
         dev::store_photon(kp.ph, L, terminated, tdisp, pdisp, have_disp);
         aa.nckpt[i] = nck;
         aa.call0[i] = c0;
+        if (count > aa.full_cap) {
+            atomicAdd(aa.over, 1);
+            count = -1;
+        }
+        aa.nfull[i] = count;
         atomicAdd(&kp.counters->calls, static_cast<unsigned long long>(L.calls));
         if (terminated) atomicAdd(&kp.counters->terminated, 1ull);
+    }
+}
+
+// The recorded rays, one thread each.
+__global__ void __launch_bounds__(128) adj_sweep(const __grid_constant__ KParams kp,
+                                                 const __grid_constant__ AdjointArgs aa) {
+    const long long n = static_cast<long long>(kp.n);
+    const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+    if (i >= n) return;
+    const int count = aa.nfull[i];
+    if (count <= 0) return;
+    if (kp.ph.phase[i] != 3) return;  // only ImageArrived rays enter the image
+    double lam = dev::pixel_adjoint(kp, aa, i);
+    for (int t = count - 1; t >= 0 && lam != 0.0; --t) {
+        const double* e = aa.full + static_cast<long long>(t) * dev::kTapeDoubles * n + i;
+        lam = dev::sweep_step(kp, aa, lam, static_cast<int>(e[0]), e[n], e[2 * n], e[3 * n], e[4 * n], e[5 * n]);
     }
 }
 
@@ -169,12 +233,11 @@ __global__ void __launch_bounds__(128, 2) adj_reverse(const __grid_constant__ KP
     const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
          i < static_cast<long long>(kp.n); i += stride) {
+        if (aa.nfull[i] >= 0) continue;  // adj_sweep's
         if (kp.ph.phase[i] != 3) continue;  // only ImageArrived rays enter the image
         const int nck = aa.nckpt[i];
         if (nck <= 0) continue;
-        const unsigned long long px = dev::observation_bin(kp.ph.theta_disp[i], -0.5 * aa.W, 0.5 * aa.W, aa.nx);
-        const unsigned long long py = dev::observation_bin(kp.ph.phi_disp[i], -0.5 * aa.H, 0.5 * aa.H, aa.ny);
-        double lam = aa.dL_dI[py * aa.nx + px];
+        double lam = dev::pixel_adjoint(kp, aa, i);
         if (lam == 0.0) continue;
         double* tape = aa.tape + static_cast<long long>(blockIdx.x * blockDim.x + threadIdx.x) * aa.K *
                                      dev::kTapeDoubles;
@@ -201,11 +264,7 @@ __global__ void __launch_bounds__(128, 2) adj_reverse(const __grid_constant__ KP
             if (m == nck - 1 && zeroed) break;  // Stokes zeroed at arrival: no dependence
             for (int t = count - 1; t >= 0; --t) {
                 const double* e = tape + static_cast<long long>(t) * dev::kTapeDoubles;
-                const int cell = static_cast<int>(e[0]);
-                const double lp = lam * e[5];
-                if (kp.emis_on) atomicAdd(aa.g_emis + cell, lp * e[2]);
-                if (kp.abs_on) atomicAdd(aa.g_abs + cell, lp * e[3] * e[4] * (-e[1]));
-                lam = lp * e[4];
+                lam = dev::sweep_step(kp, aa, lam, static_cast<int>(e[0]), e[1], e[2], e[3], e[4], e[5]);
             }
         }
     }
@@ -220,6 +279,14 @@ cudaError_t launch_adjoint_forward(const KParams& kp, const AdjointArgs& aa, int
         cudaFuncSetAttribute(adj_forward<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         adj_forward<1><<<blocks, 128, smem, stream>>>(kp, aa);
     }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_adjoint_sweep(const KParams& kp, const AdjointArgs& aa, cudaStream_t stream) {
+    const unsigned long long blocks = (kp.n + 127) / 128;
+    if (blocks == 0) return cudaSuccess;
+    if (blocks > 0x7FFFFFFFull) return cudaErrorInvalidConfiguration;
+    adj_sweep<<<static_cast<unsigned>(blocks), 128, 0, stream>>>(kp, aa);
     return cudaGetLastError();
 }
 

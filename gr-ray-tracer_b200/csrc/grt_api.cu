@@ -203,7 +203,10 @@ struct grt_ctx {
     bool has_m_abs = false, has_m_emis = false;
     // checkpointed forward / adjoint
     DevBuf<double> ckpt, tape, dLdI, g_abs, g_emis;
-    DevBuf<int> nckpt, adj_overflow;
+    DevBuf<int> nckpt, adj_overflow, adj_nfull;
+    DevBuf<double> adj_full;                 // the forward pass's transfer updates
+    int adj_full_cap = 0, adj_over = 0;
+    bool adj_stale = false;  // parameters or grid changed since: the record does not hold
     DevBuf<long long> call0;
     int adj_K = 0, adj_cap = 0;
     bool adj_ready = false;
@@ -438,6 +441,7 @@ void grt_destroy(grt_ctx* c) {
     c->m_abs.release(); c->m_emis.release();
     c->ckpt.release(); c->tape.release(); c->dLdI.release(); c->g_abs.release(); c->g_emis.release();
     c->nckpt.release(); c->adj_overflow.release(); c->call0.release();
+    c->adj_nfull.release(); c->adj_full.release();
     c->bimage.release(); c->bspectrum.release(); c->barrived.release();
     c->share_state.release(); c->calls_carry.release(); c->out_stage.release();
     if (c->host_out) cudaFreeHost(c->host_out);
@@ -461,6 +465,7 @@ grt_status grt_set_params(grt_ctx* c, const grt_params* p) {
     char buf[512];
     if (grt_params_validate(p, buf, sizeof(buf)) != GRT_OK) return fail(c, GRT_EINVAL, buf);
     c->p = *p;
+    c->adj_stale = true;
     ++c->generation;
     return GRT_OK;
 }
@@ -513,6 +518,7 @@ grt_status grt_upload_grid(grt_ctx* c, size_t nr, size_t nth, size_t nph, const 
     if (!c) return GRT_EINVAL;
     const size_t ncell = nr * nth * nph;
     ++c->generation;
+    c->adj_stale = true;
     c->grid_uploaded = true;
     c->fluid_available = false;
     c->separable = false;
@@ -1760,6 +1766,26 @@ grt_status grt_set_cell_multipliers(grt_ctx* c, const double* m_abs, const doubl
     return GRT_OK;
 }
 
+static grt::AdjointArgs adjoint_args(const grt_ctx* c) {
+    grt::AdjointArgs aa{};
+    aa.ckpt = c->ckpt.ptr;
+    aa.cap = c->adj_cap;
+    aa.K = c->adj_K;
+    aa.nckpt = c->nckpt.ptr;
+    aa.call0 = c->call0.ptr;
+    aa.overflow = c->adj_overflow.ptr;
+    aa.full = c->adj_full.ptr;
+    aa.full_cap = c->adj_full_cap;
+    aa.nfull = c->adj_nfull.ptr;
+    aa.over = c->adj_overflow.ptr + 1;
+    return aa;
+}
+
+// Transfer updates the checkpointed forward records per ray (rays of the
+// benchmark's image sample about 25 times), and the memory set aside for them.
+constexpr int64_t kRecordedSteps = 128;
+constexpr unsigned long long kRecordBytes = 4ull << 30;
+
 grt_status grt_forward_checkpointed(grt_ctx* c, int64_t K, grt_run_stats* stats) {
     if (c && c->render_pending) return rendering(c);
     if (!c) return GRT_EINVAL;
@@ -1785,7 +1811,16 @@ grt_status grt_forward_checkpointed(grt_ctx* c, int64_t K, grt_run_stats* stats)
     GRT_CUDA(c, c->ckpt.alloc(n * cap * 16), "alloc checkpoints");
     GRT_CUDA(c, c->nckpt.alloc(std::max<size_t>(n, 1)), "alloc checkpoints");
     GRT_CUDA(c, c->call0.alloc(std::max<size_t>(n, 1)), "alloc checkpoints");
-    GRT_CUDA(c, c->adj_overflow.alloc(1), "alloc checkpoints");
+    GRT_CUDA(c, c->adj_overflow.alloc(2), "alloc checkpoints");  // overflow, rays not recorded
+    GRT_CUDA(c, c->adj_nfull.alloc(std::max<size_t>(n, 1)), "alloc checkpoints");
+    // the record of every ray's transfer updates, as far as the memory set
+    // aside for it goes; rays with more updates are traced again by the adjoint
+    c->adj_full_cap = static_cast<int>(std::min<unsigned long long>(
+        std::min<int64_t>(p.max_steps, kRecordedSteps), kRecordBytes / (48ull * std::max<size_t>(n, 1))));
+    if (c->adj_full.alloc(n * c->adj_full_cap * 6) != cudaSuccess) {
+        cudaGetLastError();
+        c->adj_full_cap = 0;
+    }
     GRT_CUDA(c, c->tape.alloc(static_cast<size_t>(blocks) * threads * K * 6), "alloc tape");
     c->adj_K = static_cast<int>(K);
     c->adj_cap = static_cast<int>(cap);
@@ -1798,28 +1833,24 @@ grt_status grt_forward_checkpointed(grt_ctx* c, int64_t K, grt_run_stats* stats)
     grt::KParams kp = make_kparams(c);
     kp.step0 = 0;
     kp.budget = p.max_steps;
-    grt::AdjointArgs aa{};
-    aa.ckpt = c->ckpt.ptr;
-    aa.cap = c->adj_cap;
-    aa.K = c->adj_K;
-    aa.nckpt = c->nckpt.ptr;
-    aa.call0 = c->call0.ptr;
-    aa.overflow = c->adj_overflow.ptr;
+    grt::AdjointArgs aa = adjoint_args(c);
     GRT_CUDA(c, cudaMemsetAsync(c->counters.ptr, 0, sizeof(grt::KCounters), c->stream), "memset");
-    GRT_CUDA(c, cudaMemsetAsync(c->adj_overflow.ptr, 0, sizeof(int), c->stream), "memset");
+    GRT_CUDA(c, cudaMemsetAsync(c->adj_overflow.ptr, 0, 2 * sizeof(int), c->stream), "memset");
     GRT_CUDA(c, cudaEventRecord(c->ev0, c->stream), "event");
     cudaError_t e = grt::launch_adjoint_forward(kp, aa, blocks, trace_smem(c), c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "adjoint forward launch");
     GRT_CUDA(c, cudaEventRecord(c->ev1, c->stream), "event");
     GRT_CUDA(c, cudaMemcpyAsync(c->host_counters, c->counters.ptr, sizeof(grt::KCounters), cudaMemcpyDeviceToHost,
                                 c->stream), "D2H counters");
-    int overflow = 0;
-    GRT_CUDA(c, cudaMemcpyAsync(&overflow, c->adj_overflow.ptr, sizeof(int), cudaMemcpyDeviceToHost, c->stream),
+    int overflow[2] = {0, 0};
+    GRT_CUDA(c, cudaMemcpyAsync(overflow, c->adj_overflow.ptr, sizeof(overflow), cudaMemcpyDeviceToHost, c->stream),
              "D2H");
     GRT_CUDA(c, cudaStreamSynchronize(c->stream), "adjoint forward");
     float ms = 0.0f;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);
-    if (overflow) return fail(c, GRT_ECUDA, "checkpoint capacity exceeded");
+    if (overflow[0]) return fail(c, GRT_ECUDA, "checkpoint capacity exceeded");
+    c->adj_over = overflow[1];
+    c->adj_stale = false;
     const grt::KCounters& k = *c->host_counters;
     st.photon_calls = k.calls;
     st.n_terminated = k.terminated + c->initial_terminated;
@@ -1850,13 +1881,7 @@ grt_status grt_adjoint_image_I(grt_ctx* c, const double* dL_dI, double* g_abs, d
         grt::KParams kp = make_kparams(c);
         kp.step0 = 0;
         kp.budget = p.max_steps;
-        grt::AdjointArgs aa{};
-        aa.ckpt = c->ckpt.ptr;
-        aa.cap = c->adj_cap;
-        aa.K = c->adj_K;
-        aa.nckpt = c->nckpt.ptr;
-        aa.call0 = c->call0.ptr;
-        aa.overflow = c->adj_overflow.ptr;
+        grt::AdjointArgs aa = adjoint_args(c);
         aa.dL_dI = c->dLdI.ptr;
         aa.nx = p.image_nx;
         aa.ny = p.image_ny;
@@ -1868,7 +1893,11 @@ grt_status grt_adjoint_image_I(grt_ctx* c, const double* dL_dI, double* g_abs, d
         const int threads = 128;
         const size_t tape_threads = c->tape.count / (static_cast<size_t>(c->adj_K) * 6);
         const int blocks = static_cast<int>(std::max<size_t>(1, tape_threads / threads));
-        cudaError_t e = grt::launch_adjoint_reverse(kp, aa, blocks, trace_smem(c), c->stream);
+        cudaError_t e = cudaSuccess;
+        if (c->adj_stale) e = cudaMemsetAsync(c->adj_nfull.ptr, 0xFF, c->n * sizeof(int), c->stream);
+        else e = grt::launch_adjoint_sweep(kp, aa, c->stream);
+        if (e == cudaSuccess && (c->adj_over > 0 || c->adj_stale))
+            e = grt::launch_adjoint_reverse(kp, aa, blocks, trace_smem(c), c->stream);
         if (e != cudaSuccess) return cuda_fail(c, e, "adjoint reverse launch");
     }
     int overflow = 0;

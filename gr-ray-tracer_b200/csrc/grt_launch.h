@@ -105,7 +105,13 @@ struct AdjointArgs {
     double W, H;
     double* g_abs;             // [ncell] dL/dm_abs (accumulated)
     double* g_emis;            // [ncell] dL/dm_emis
-    double* tape;              // [threads][K][6]
+    double* tape;              // [threads][K][6] of a recomputed segment
+    // the forward pass's own record of each ray's transfer updates: field f of
+    // entry e of queue position q at full[(e * 6 + f) * n + q]
+    double* full;
+    int full_cap;              // entries a ray can keep (0: no record)
+    int* nfull;                // [n] entries kept, -1 when the ray had more
+    int* over;                 // rays with nfull -1
 };
 
 // Camera plane basis of integrate_cart_ks.hpp:97-107 with host libm, plus the
@@ -186,9 +192,11 @@ inline size_t dev_trace_smem_bytes(int integrator, int threads, bool separable, 
     return n * sizeof(double);
 }
 
-// Adjoint pass: checkpointed forward trace and reverse sweep, 128-thread blocks.
+// Adjoint pass: checkpointed forward trace, the sweep of the rays it recorded and
+// the reverse pass of the others, 128-thread blocks.
 cudaError_t launch_adjoint_forward(const KParams& kp, const AdjointArgs& aa, int blocks, size_t smem,
                                    cudaStream_t stream);
+cudaError_t launch_adjoint_sweep(const KParams& kp, const AdjointArgs& aa, cudaStream_t stream);
 cudaError_t launch_adjoint_reverse(const KParams& kp, const AdjointArgs& aa, int blocks, size_t smem,
                                    cudaStream_t stream);
 
