@@ -1172,7 +1172,8 @@ cudaError_t reset_trace(const grt_ctx* c, int chunks = 1) {
 }
 
 size_t trace_smem(const grt_ctx* c) {
-    return grt::dev_trace_smem_bytes(c->p.integrator, 128, c->fluid_available && c->separable, c->nr, c->nth, c->nph);
+    return grt::dev_trace_smem_bytes(c->p.integrator, 128, c->fluid_available && c->separable, c->nr, c->nth, c->nph,
+                                     c->p.mode == GRT_MODE_DISK);
 }
 
 // steps_done of a single-launch run (termination_percent = 1): the reference

@@ -183,11 +183,16 @@ inline void set_axis_lookup(KGrid& g, const double* ra, const double* ta, const 
     g.even = even ? 1 : 0;
 }
 
-// Dynamic shared memory of a trace launch: the stage slots for RK45 (6*7
-// doubles per thread: k1..k5, then the state) plus the separable axes and
-// their half-spans (2*(nr+nth+nph)).
-inline size_t dev_trace_smem_bytes(int integrator, int threads, bool separable, int nr, int nth, int nph) {
-    size_t n = integrator == 1 ? static_cast<size_t>(6 * 7) * threads : 0;
+// Stage slots of an RK45 block: the disk mode's rolled error norm keeps the
+// state in a sixth (rk45_attempt).
+__host__ __device__ constexpr int stage_slots(bool disk) { return disk ? 6 : 5; }
+
+// Dynamic shared memory of a trace launch: the stage slots for RK45 (7 doubles
+// per thread and slot) plus the separable axes and their half-spans
+// (2*(nr+nth+nph)).
+inline size_t dev_trace_smem_bytes(int integrator, int threads, bool separable, int nr, int nth, int nph,
+                                   bool disk = false) {
+    size_t n = integrator == 1 ? static_cast<size_t>(stage_slots(disk) * 7) * threads : 0;
     if (separable) n += 2 * static_cast<size_t>(nr + nth + nph);
     return n * sizeof(double);
 }

@@ -255,12 +255,12 @@ static __constant__ double kFehlbergA[5][5] = {
 constexpr int kTraceThreads = 128;
 
 // Per-thread slots in shared memory: the stage derivatives k1..k5 (slots
-// 0..4) and, for the rolled error norm, k6 in place of k2 in slot 1 and the
-// state in slot 5.  [6][7][kTraceThreads] doubles,
+// 0..4) and, for the rolled error norm (WIDE false), k6 in place of k2 in slot
+// 1 and the state in a sixth slot (dev_trace_smem_bytes gives every kernel but
+// the disk mode's five).  [5 or 6][7][kTraceThreads] doubles,
 // thread-contiguous so a warp's accesses are conflict-free; base already
 // points at this thread's column, so a slot is a constant offset from it.
 // k1 stays there across the retries of one call.
-constexpr int kStageSlots = 6;
 struct KStore {
     double* base;
     GRT_DEV double& at(int j, int c) const { return base[(j * 7 + c) * kTraceThreads]; }
@@ -293,7 +293,10 @@ GRT_DEV void larger_ratio(double& n, double& sc, double m, double sd) {
 // the warp stays converged on the same code -- and the derivatives live in
 // shared memory (KStore), which keeps registers for the right-hand side.
 // Each stage input is summed over j = 1..t-1 left to right, the reference's
-// association; for the first stage, dt*(a21 k1) equals the reference's
+// association, in a rolled loop: as straight-line code per stage it ran slower
+// on every workload, a lone warp's too (256 rays 0.421 / 0.443 ms, 4.76e6 33.8 /
+// 35.8; code that runs once an attempt is fetched anew each time);
+// for the first stage, dt*(a21 k1) equals the reference's
 // (dt*a21)*k1 because a21 = 1/4 is a power of two.
 //
 // The error norm is max_c RN(n_c / sc_c).  Rounding is monotone, so it equals
@@ -326,11 +329,30 @@ GRT_DEV int rk45_attempt(const KParams& kp, double s[8], double* dl, int need_k1
             const double a0 = kFehlbergA[st][0];
 #pragma unroll
             for (int c = 0; c < 7; ++c) acc[c] = a0 * kk.at(0, c);
-#pragma unroll 1
-            for (int j = 1; j <= st; ++j) {
-                const double aj = kFehlbergA[st][j];
+            if constexpr (WIDE) {
+                // each pass loads the next derivative while it adds this one
+                double kj[7], aj = kFehlbergA[st][1];
 #pragma unroll
-                for (int c = 0; c < 7; ++c) acc[c] = acc[c] + aj * kk.at(j, c);
+                for (int c = 0; c < 7; ++c) kj[c] = kk.at(1, c);
+#pragma unroll 2
+                for (int j = 1; j <= st; ++j) {
+                    const int next = min(j + 1, 4);  // the last slot
+                    const double an = kFehlbergA[st][next];
+#pragma unroll
+                    for (int c = 0; c < 7; ++c) {
+                        const double kn = kk.at(next, c);
+                        acc[c] = acc[c] + aj * kj[c];
+                        kj[c] = kn;
+                    }
+                    aj = an;
+                }
+            } else {
+#pragma unroll 1
+                for (int j = 1; j <= st; ++j) {
+                    const double aj = kFehlbergA[st][j];
+#pragma unroll
+                    for (int c = 0; c < 7; ++c) acc[c] = acc[c] + aj * kk.at(j, c);
+                }
             }
 #pragma unroll
             for (int c = 0; c < 7; ++c) t[sidx(c)] = s[sidx(c)] + dt * acc[c];
@@ -1052,11 +1074,11 @@ GRT_DEV bool run_stopped(const KParams& kp) {
 
 // Shared-memory layout of a trace block: [stage slots (RK45)] [axes and
 // half-spans of a separable grid].  Returns the staged pointers.
-GRT_DEV void stage_grid(const KParams& kp, double* smem, int integrator, Axes& ax, KStore& kk) {
+GRT_DEV void stage_grid(const KParams& kp, double* smem, int integrator, Axes& ax, KStore& kk, int slots = 5) {
     const KGrid& G = kp.grid;
     double* p = smem;
     kk.base = p + threadIdx.x;
-    if (integrator == 1) p += kStageSlots * 7 * kTraceThreads;
+    if (integrator == 1) p += slots * 7 * kTraceThreads;
     if (G.available && G.separable) {
         double* r = p;
         double* th = r + G.nr;

@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(128, MINB) GRT_TRACE_KERNEL(const __grid_const
     if (kp.n_prior && dev::run_stopped(kp)) return;
     dev::Axes ax;
     dev::KStore kk;
-    dev::stage_grid(kp, smem, INTEGRATOR, ax, kk);
+    dev::stage_grid(kp, smem, INTEGRATOR, ax, kk, stage_slots(LEG == 3));
     dev::trace_body<INTEGRATOR, GRT_TRACE_RHS(MINB), false, SHARE, LEG>(kp, ax, kk);
 }
 
