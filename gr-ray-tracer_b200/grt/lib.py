@@ -178,7 +178,20 @@ def trace_device_noalloc(params: Params, grid: DeviceGrid, photons: PhotonSoA, n
     return st.as_dict()
 
 
+def _on_device(a) -> bool:
+    """Whether a is a torch tensor in device memory; one the library can read or write in place must be
+    contiguous float64."""
+    if not getattr(a, "is_cuda", False):
+        return False
+    if str(a.dtype) != "torch.float64" or not a.is_contiguous():
+        raise TypeError("device tensors must be contiguous float64")
+    return True
+
+
 def _dp(a):
+    """double* of a float64 numpy array or device tensor."""
+    if _on_device(a):
+        return C.cast(a.data_ptr(), C.POINTER(C.c_double))
     return a.ctypes.data_as(C.POINTER(C.c_double))
 
 
@@ -325,8 +338,9 @@ class Context:
 
     # ---- differentiable radiative transfer ----
     def set_cell_multipliers(self, m_abs=None, m_emis=None):
-        """Per-cell multipliers on dtau and dI (arrays of the grid's shape; None = 1)."""
-        self._mult = [None if m is None else np.ascontiguousarray(m, dtype=np.float64).ravel()
+        """Per-cell multipliers on dtau and dI (arrays of the grid's shape, or
+        contiguous float64 CUDA tensors that are complete; None = 1)."""
+        self._mult = [m if m is None or _on_device(m) else np.ascontiguousarray(m, dtype=np.float64).ravel()
                       for m in (m_abs, m_emis)]
         self._check(self.lib.grt_set_cell_multipliers(self._h, *[_dp(m) if m is not None else None
                                                                   for m in self._mult]))
@@ -345,6 +359,15 @@ class Context:
         ge = np.zeros(int(np.prod(grid_shape)))
         self._check(self.lib.grt_adjoint_image_I(self._h, _dp(g), _dp(ga), _dp(ge)))
         return ga.reshape(grid_shape), ge.reshape(grid_shape)
+
+    def adjoint_image_I_device(self, dL_dimage_I, g_abs, g_emis):
+        """adjoint_image_I on contiguous float64 CUDA tensors: reads the complete
+        dL_dimage_I, fills g_abs and g_emis before it returns."""
+        if tuple(dL_dimage_I.shape) != (self.params.image_ny, self.params.image_nx):
+            raise ValueError(f"dL/dimage_I must have shape {(self.params.image_ny, self.params.image_nx)}")
+        if not all(_on_device(t) for t in (dL_dimage_I, g_abs, g_emis)):
+            raise TypeError("adjoint_image_I_device takes device tensors")
+        self._check(self.lib.grt_adjoint_image_I(self._h, _dp(dL_dimage_I), _dp(g_abs), _dp(g_emis)))
 
     def run(self) -> dict:
         st = RunStats()

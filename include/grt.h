@@ -473,8 +473,8 @@ grt_status grt_render_wait(grt_ctx* ctx, grt_run_stats* stats);
  * dtau = m_abs[cell] * ComputeOpticalDepthIncrement(...) and
  * dI = m_emis[cell] * ComputeEmissivityIncrement(...)
  * (radiative_transfer.hpp:61-96), so the gradient below is exact for any
- * user body.  Arrays are host float64 of length nr*ntheta*nphi (C order of
- * the grid); NULL switches that multiplier off (all ones).  Applies to every
+ * user body.  Arrays are float64 of length nr*ntheta*nphi (C order of
+ * the grid), in host memory or on the device (complete when the call is made); NULL switches that multiplier off (all ones).  Applies to every
  * later trace (grt_run, grt_render_graph, the checkpointed forward).
  */
 grt_status grt_set_cell_multipliers(grt_ctx* ctx, const double* m_abs, const double* m_emis);
@@ -487,11 +487,13 @@ grt_status grt_set_cell_multipliers(grt_ctx* ctx, const double* m_abs, const dou
 grt_status grt_forward_checkpointed(grt_ctx* ctx, int64_t checkpoint_interval, grt_run_stats* stats);
 
 /*
- * Adjoint of the last grt_forward_checkpointed: given dL/d(image_I) (host,
- * [image_ny][image_nx], the binning of grt_get_image_products), write
- * dL/dm_abs and dL/dm_emis (host, [nr*ntheta*nphi]; either may be NULL).
- * Each ray's segments are recomputed from its checkpoints (bit-identical to
- * the forward pass) and its radiative-transfer updates swept backwards.
+ * Adjoint of the last grt_forward_checkpointed: given dL/d(image_I)
+ * ([image_ny][image_nx], the binning of grt_get_image_products), write
+ * dL/dm_abs and dL/dm_emis ([nr*ntheta*nphi]; either may be NULL); each array
+ * in host memory or on the device.  The radiative-transfer updates that the
+ * forward pass recorded are swept backwards; a ray with more of them than the
+ * record holds is traced again from its checkpoints (bit-identical to the
+ * forward pass).  The gradients are complete when the call returns.
  */
 grt_status grt_adjoint_image_I(grt_ctx* ctx, const double* dL_dimage_I, double* dL_dm_abs, double* dL_dm_emis);
 
