@@ -207,35 +207,31 @@ GRT_DEV int store_all(const KParams& kp, const Lane& L, int terminated, double t
 }
 
 // integrate_cart_ks.hpp:142-155.  One right-hand-side site inside a stage
-// loop (kept rolled: a fully unrolled step overflows the instruction cache);
-// only the running weighted sum ((k1 + 2 k2) + 2 k3) + k4 is kept, which adds
-// the stages in the reference's order.  Stage inputs s + (c dt) k with
-// c in {1/2, 1/2, 1} round exactly like the reference's s + c*dt*k.
+// loop (kept rolled: a fully unrolled step overflows the instruction cache,
+// 2.146 against 2.111 ms for 4,096 rays), without a branch: with a "0th"
+// derivative of -0.0 the first stage is the others' code (s + 1 * (-0.0) = s
+// and -0.0 + k = k, signed zeros included), and a warp alone on its scheduler
+// waits for no decision between the stages (2.457 ms with one).  Only the
+// running weighted sum ((k1 + 2 k2) + 2 k3) + k4 is kept, which adds the stages
+// in the reference's order.  Stage inputs s + (c dt) k with c in
+// {1/2, 1/2, 1} round exactly like the reference's s + c*dt*k.
 template <class RHS>
 GRT_DEV void rk4_step(double s[8], double dt, const KParams& kp, int fast) {
     double t[8];
     V7 k, sum;
     t[4] = s[4];
+#pragma unroll
+    for (int c = 0; c < 7; ++c) k.v[c] = sum.v[c] = -0.0;
+    double cdt = 1.0, w = 1.0;
 #pragma unroll 1
     for (int st = 0; st < 4; ++st) {
-        if (st == 0) {
 #pragma unroll
-            for (int c = 0; c < 7; ++c) t[sidx(c)] = s[sidx(c)];
-        } else {
-            const double cdt = (st == 3) ? dt : 0.5 * dt;
-#pragma unroll
-            for (int c = 0; c < 7; ++c) t[sidx(c)] = s[sidx(c)] + cdt * k.v[c];
-        }
+        for (int c = 0; c < 7; ++c) t[sidx(c)] = s[sidx(c)] + cdt * k.v[c];
         k = RHS::eval(t, kp, fast);
-        if (st == 0) {
-            sum = k;
-        } else if (st == 3) {
 #pragma unroll
-            for (int c = 0; c < 7; ++c) sum.v[c] = sum.v[c] + k.v[c];
-        } else {
-#pragma unroll
-            for (int c = 0; c < 7; ++c) sum.v[c] = sum.v[c] + 2.0 * k.v[c];
-        }
+        for (int c = 0; c < 7; ++c) sum.v[c] = sum.v[c] + w * k.v[c];
+        cdt = st == 2 ? dt : 0.5 * dt;
+        w = st == 2 ? 1.0 : 2.0;
     }
     const double h6 = dt / 6.0;
 #pragma unroll
