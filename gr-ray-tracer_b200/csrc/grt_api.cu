@@ -183,6 +183,7 @@ struct grt_ctx {
     // tile orders of the image-mode queue (queue position -> index): over
     // photon slots and over the geodesics of channel groups
     DevBuf<unsigned> order_ph, order_geo;
+    DevBuf<unsigned> screen_scratch;  // cells, ranks and counts behind the order of a random screen
     // layout the tile orders were built for (image slot starts and widths,
     // group starts and widths): a new image set with the same layout reuses them
     std::vector<unsigned long long> order_layout;
@@ -355,7 +356,7 @@ grt::KParams make_kparams(const grt_ctx* c) {
         k.n = c->geodesics;
         k.share_state = c->share_state.ptr;
     }
-    if (k.image_mode && c->have_images && !c->random_screen)
+    if (k.image_mode && c->have_images)
         k.order = k.ngroups > 0 ? (c->order_geo_ok ? c->order_geo.ptr : nullptr)
                                 : (c->order_ph_ok ? c->order_ph.ptr : nullptr);
     k.calls_carry = c->calls_carry.ptr;
@@ -446,7 +447,7 @@ void grt_destroy(grt_ctx* c) {
         if (e) cudaEventDestroy(e);
     c->images_dev.release(); c->image_start_dev.release();
     c->group_qstart_dev.release(); c->group_chan_dev.release(); c->chan_img_dev.release();
-    c->order_ph.release(); c->order_geo.release(); c->sm_claims.release();
+    c->order_ph.release(); c->order_geo.release(); c->sm_claims.release(); c->screen_scratch.release();
     c->m_abs.release(); c->m_emis.release();
     c->ckpt.release(); c->tape.release(); c->dLdI.release(); c->g_abs.release(); c->g_emis.release();
     c->nckpt.release(); c->adj_overflow.release(); c->call0.release();
@@ -875,7 +876,8 @@ grt_status set_tile_orders(grt_ctx* c, const std::vector<unsigned long long>& st
     layout.push_back(~0ull);
     layout.insert(layout.end(), qstart.begin(), qstart.end());
     for (size_t g = 0; g + 1 < qstart.size(); ++g) layout.push_back(c->images[chan[gchan[g]]].nx);
-    const bool usable = !c->random_screen && c->n < (1ull << 32);
+    if (c->random_screen) return GRT_OK;  // set_screen_order, once the rays are there
+    const bool usable = c->n < (1ull << 32);
     if (usable && layout == c->order_layout && c->order_ph_ok && (qstart.empty() || c->order_geo_ok))
         return GRT_OK;  // same layout: the orders on the device still hold
     c->order_ph_ok = c->order_geo_ok = false;
@@ -901,6 +903,34 @@ grt_status set_tile_orders(grt_ctx* c, const std::vector<unsigned long long>& st
         c->order_geo_ok = ord.size() == c->geodesics;
     }
     c->order_layout = std::move(layout);
+    return GRT_OK;
+}
+
+// The queue order of a random screen's rays (launch_screen_order), from the
+// positions the initialisation has just enqueued.
+grt_status set_screen_order(grt_ctx* c) {
+    c->order_ph_ok = c->order_geo_ok = false;
+    c->order_layout.clear();
+    if (c->n >= (1ull << 32)) return GRT_OK;
+    grt::ScreenOrderArgs a{};
+    a.n = c->n;
+    a.log_side = 0;
+    while (a.log_side < 8 && (8ull << (2 * a.log_side)) < c->n) ++a.log_side;
+    if (c->order_ph.alloc(c->n) != cudaSuccess ||
+        c->screen_scratch.alloc(2 * c->n + (1ull << (2 * a.log_side)) + 1) != cudaSuccess) {
+        cudaGetLastError();  // no memory for it: the rays are traced in the order they were drawn
+        return GRT_OK;
+    }
+    a.u = c->ph.f[15].ptr;  // theta_disp, phi_disp
+    a.v = c->ph.f[16].ptr;
+    a.W = c->images[0].camera_width;
+    a.H = c->images[0].camera_height;
+    a.cell = c->screen_scratch.ptr;
+    a.rank = a.cell + c->n;
+    a.count = a.rank + c->n;
+    a.order = c->order_ph.ptr;
+    GRT_CUDA(c, grt::launch_screen_order(a, c->stream), "screen order");
+    c->order_ph_ok = true;
     return GRT_OK;
 }
 
@@ -999,7 +1029,8 @@ grt_status set_image_set(grt_ctx* c, const grt_image_spec* specs, size_t nimages
         const grt_status os = set_tile_orders(c, start, {}, {}, {});
         if (os != GRT_OK) return os;
     }
-    return launch_image_inits(c);
+    const grt_status is = launch_image_inits(c);
+    return is == GRT_OK && random_screen ? set_screen_order(c) : is;
 }
 
 // Launch-wide part of a build_observation_products (observation.hpp:31-84) launch.

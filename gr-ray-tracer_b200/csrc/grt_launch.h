@@ -79,6 +79,18 @@ struct ProductsSet {
     ProductsImage img[kProductsMaxImages];
 };
 
+// Queue order of n rays at screen positions (u, v) in a W x H window: by cells
+// of a 2^log_side x 2^log_side screen grid (log_side <= 8).
+struct ScreenOrderArgs {
+    const double *u, *v;           // [n]
+    double W, H;
+    unsigned long long n;          // < 2^32
+    int log_side;
+    int pad;
+    unsigned *cell, *rank, *order; // [n]
+    unsigned* count;               // [4^log_side + 1]
+};
+
 // Strided gather of an output step's photon fields (write_output_step):
 // elements src[k][j * stride], j < count, of field k packed at dst + dst_off[k].
 constexpr int kGatherMaxFields = 40;  // a selection's fields, "all" after 20 names included
@@ -233,6 +245,7 @@ cudaError_t launch_generate_pending(const KParams& kp, int sm_count, size_t smem
 cudaError_t launch_trace(const KParams& kp, bool mixed, int leg, int integrator, int sm_count, int blocks_per_sm,
                          size_t smem, cudaStream_t stream);
 cudaError_t launch_init_image(const InitImageArgs& args, cudaStream_t stream);
+cudaError_t launch_screen_order(const ScreenOrderArgs& a, cudaStream_t stream);
 cudaError_t launch_init_disk(const DiskInitArgs& a, cudaStream_t stream);
 // Fills block0 / blocks of `set` and launches it.
 cudaError_t launch_image_products(ProductsSet& set, cudaStream_t stream);
