@@ -291,8 +291,9 @@ GRT_DEV void larger_ratio(double& n, double& sc, double m, double sd) {
 // Each stage input is summed over j = 1..t-1 left to right, the reference's
 // association, in a rolled loop: as straight-line code per stage it ran slower
 // on every workload, a lone warp's too (256 rays 0.421 / 0.443 ms, 4.76e6 33.8 /
-// 35.8; code that runs once an attempt is fetched anew each time);
-// for the first stage, dt*(a21 k1) equals the reference's
+// 35.8; code that runs once an attempt is fetched anew each time).  Without
+// branches (WIDE false) the disk mode gains 1% and the image kernels lose 2%.
+// For the first stage, dt*(a21 k1) equals the reference's
 // (dt*a21)*k1 because a21 = 1/4 is a power of two.
 //
 // The error norm is max_c RN(n_c / sc_c).  Rounding is monotone, so it equals
@@ -317,7 +318,22 @@ GRT_DEV int rk45_attempt(const KParams& kp, double s[8], double* dl, int need_k1
     t[4] = s[4];
 #pragma unroll 1
     for (int st = need_k1 ? -1 : 0; st < 5; ++st) {
-        if (st < 0) {
+        if constexpr (!WIDE) {
+            // one path for every stage, the call's own k1 (no terms: s + 1 *
+            // (-0.0)) included
+            const double h = st < 0 ? 1.0 : dt;
+            double acc[7];
+#pragma unroll
+            for (int c = 0; c < 7; ++c) acc[c] = -0.0;
+#pragma unroll 1
+            for (int j = 0; j <= st; ++j) {
+                const double aj = kFehlbergA[st][j];
+#pragma unroll
+                for (int c = 0; c < 7; ++c) acc[c] = acc[c] + aj * kk.at(j, c);
+            }
+#pragma unroll
+            for (int c = 0; c < 7; ++c) t[sidx(c)] = s[sidx(c)] + h * acc[c];
+        } else if (st < 0) {
 #pragma unroll
             for (int c = 0; c < 7; ++c) t[sidx(c)] = s[sidx(c)];
         } else {
@@ -325,30 +341,21 @@ GRT_DEV int rk45_attempt(const KParams& kp, double s[8], double* dl, int need_k1
             const double a0 = kFehlbergA[st][0];
 #pragma unroll
             for (int c = 0; c < 7; ++c) acc[c] = a0 * kk.at(0, c);
-            if constexpr (WIDE) {
-                // each pass loads the next derivative while it adds this one
-                double kj[7], aj = kFehlbergA[st][1];
+            // each pass loads the next derivative while it adds this one
+            double kj[7], aj = kFehlbergA[st][1];
 #pragma unroll
-                for (int c = 0; c < 7; ++c) kj[c] = kk.at(1, c);
+            for (int c = 0; c < 7; ++c) kj[c] = kk.at(1, c);
 #pragma unroll 2
-                for (int j = 1; j <= st; ++j) {
-                    const int next = min(j + 1, 4);  // the last slot
-                    const double an = kFehlbergA[st][next];
+            for (int j = 1; j <= st; ++j) {
+                const int next = min(j + 1, 4);  // the last slot
+                const double an = kFehlbergA[st][next];
 #pragma unroll
-                    for (int c = 0; c < 7; ++c) {
-                        const double kn = kk.at(next, c);
-                        acc[c] = acc[c] + aj * kj[c];
-                        kj[c] = kn;
-                    }
-                    aj = an;
+                for (int c = 0; c < 7; ++c) {
+                    const double kn = kk.at(next, c);
+                    acc[c] = acc[c] + aj * kj[c];
+                    kj[c] = kn;
                 }
-            } else {
-#pragma unroll 1
-                for (int j = 1; j <= st; ++j) {
-                    const double aj = kFehlbergA[st][j];
-#pragma unroll
-                    for (int c = 0; c < 7; ++c) acc[c] = acc[c] + aj * kk.at(j, c);
-                }
+                aj = an;
             }
 #pragma unroll
             for (int c = 0; c < 7; ++c) t[sidx(c)] = s[sidx(c)] + dt * acc[c];
