@@ -1150,8 +1150,8 @@ grt_status prepare_trace_buffers(grt_ctx* c, unsigned long long queue) {
 // packets live from a few calls to hundreds and a warp keeps its lanes filled
 // from the queue, so residency does not matter; the longest packets' latency
 // and the instruction cache do.  Trace ms at 2 / 3 / 4 blocks: 1.3e4 packets
-// 2.85 / 3.23 / 4.16, 1.1e5 4.70 / 5.39 / 6.81, 3.4e5 9.08 / 9.29 / 11.0, 5.7e5
-// 14.2 / 13.8 / 15.9, 2.07e6 45.2 / 42.4 / 46.2: 3 above eight packets for
+// 2.77 / 2.90 / 3.77, 1.1e5 4.50 / 4.84 / 6.02, 3.4e5 8.70 / 8.50 / 9.75, 5.7e5
+// 13.5 / 12.6 / 14.2, 2.07e6 42.5 / 38.0 / 41.5: 3 above eight packets for
 // every lane of 2 blocks, 2 below.
 int trace_blocks_per_sm(const grt_ctx* c, unsigned long long queue) {
     if (c->lc.blocks_per_sm) return c->lc.blocks_per_sm;

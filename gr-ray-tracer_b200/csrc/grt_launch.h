@@ -155,8 +155,8 @@ inline KImage make_kimage(double theta, double phi, double distance, double widt
 // mixes rays on their first and last calls.  Trace ms at 8 / 32: 64 images
 // (4.76e6 rays) 50.3 / 40.0, 509 x 283 random screen 2.61 / 2.20, 256 x 256
 // (all rays resident) 1.20 / 1.18.  Disk packets live from a few calls to
-// hundreds, and waiting for the longest leaves the warp empty: at 1 / 4 / 8 /
-// 32, 2.07e6 packets 62.3 / 62.1 / 65.2 / 138 (3 blocks/SM 60.8 / 61.1 / 63.9).
+// hundreds, and waiting for the longest leaves the warp empty: at 1 / 4 / 8,
+// 2.07e6 packets 38.2 / 38.0 / 39.4 (and more than twice that at 32).
 inline int default_refill(int image_mode) { return image_mode ? 32 : 4; }
 
 // Whether the spin a and mass M admit the reciprocal-quotient right-hand side

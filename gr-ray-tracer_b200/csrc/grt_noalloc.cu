@@ -106,13 +106,25 @@ __global__ void noalloc_count_terminated(const uint8_t* term, unsigned long long
     if ((threadIdx.x & 31) == 0 && c) atomicAdd(out, c);
 }
 
-template <int INTEGRATOR>
-__global__ void __launch_bounds__(128, 4) trace_noalloc(const __grid_constant__ grt::KParams kp) {
+// B: resident blocks per SM, i.e. the register cap.  With 2 the kernel is the
+// latency-bound form of the context's (Fp64RhsT<true>), for launches whose
+// photons all fit in its lanes: a call on 10,000 rays 1.10 / 0.61 ms at 4 / 2.
+template <int INTEGRATOR, int B>
+__global__ void __launch_bounds__(128, B) trace_noalloc(const __grid_constant__ grt::KParams kp) {
     extern __shared__ double smem[];
     grt::dev::Axes ax;
     grt::dev::KStore kk;
     grt::dev::stage_grid(kp, smem, INTEGRATOR, ax, kk);
-    grt::dev::trace_body<INTEGRATOR, grt::dev::Fp64RhsT<>, true>(kp, ax, kk);
+    grt::dev::trace_body<INTEGRATOR, grt::dev::Fp64RhsT<B == 2>, true>(kp, ax, kk);
+}
+
+template <int INTEGRATOR, int B>
+cudaError_t launch_noalloc(const grt::KParams& kp, int sms, size_t smem, cudaStream_t stream) {
+    cudaError_t e = cudaFuncSetAttribute(trace_noalloc<INTEGRATOR, B>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
+    trace_noalloc<INTEGRATOR, B><<<sms * B, 128, smem, stream>>>(kp);
+    return cudaGetLastError();
 }
 
 grt_status set_err(char* err, size_t len, const char* msg) {
@@ -292,6 +304,16 @@ extern "C" grt_status grt_trace_device_noalloc(const grt_params* p, const grt_de
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // every photon in a lane of 2 blocks per SM: the latency-bound form, its
+    // warps' first claims spread over the SMs (KParams::sm_quota) when the
+    // scratch has room for their counters behind the grid's axes
+    const bool resident = n <= static_cast<uint64_t>(sms) * 2 * 128;
+    const size_t claims_offset = kAxesOffset + 16 * (nr + nth + nph);
+    if (resident && n && claims_offset + grt::kSmClaimSlots * sizeof(unsigned) <= kNoallocScratchBytes) {
+        kp.sm_claims = reinterpret_cast<unsigned*>(static_cast<unsigned char*>(scratch) + claims_offset);
+        const unsigned long long claims = (n + kp.grab - 1) / kp.grab;
+        kp.sm_quota = static_cast<unsigned>((claims + sms - 1) / sms);
+    }
     const uint64_t interval = p->output_interval ? p->output_interval : 1;
     const bool single = p->termination_percent >= 1.0;
     int64_t step = 0, steps_done = 0;
@@ -310,12 +332,13 @@ extern "C" grt_status grt_trace_device_noalloc(const grt_params* p, const grt_de
                             (1ull << 20);
         grt::KCounters host;
         cudaError_t e = cudaMemsetAsync(counters, 0, sizeof(grt::KCounters), stream);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(p->integrator == GRT_RK4 ? trace_noalloc<0> : trace_noalloc<1>,
-                                                      cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if (e == cudaSuccess && kp.sm_quota)
+            e = cudaMemsetAsync(kp.sm_claims, 0, grt::kSmClaimSlots * sizeof(unsigned), stream);
         if (e == cudaSuccess) {
-            if (p->integrator == GRT_RK4) trace_noalloc<0><<<sms * 4, 128, smem, stream>>>(kp);
-            else trace_noalloc<1><<<sms * 4, 128, smem, stream>>>(kp);
-            e = cudaGetLastError();
+            if (p->integrator == GRT_RK4)
+                e = resident ? launch_noalloc<0, 2>(kp, sms, smem, stream) : launch_noalloc<0, 4>(kp, sms, smem, stream);
+            else
+                e = resident ? launch_noalloc<1, 2>(kp, sms, smem, stream) : launch_noalloc<1, 4>(kp, sms, smem, stream);
         }
         if (e == cudaSuccess) e = cudaMemcpyAsync(&host, counters, sizeof(host), cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
