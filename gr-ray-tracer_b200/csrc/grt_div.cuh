@@ -54,6 +54,12 @@ __device__ __forceinline__ double div_by(double a, double b, double y) {
     return fma(-n, y, q0);
 }
 
+// v / 2 for a normal v whose half is normal, on the integer pipe.  Zeros,
+// subnormals and the smallest normals give a negative number or NaN.
+__device__ __forceinline__ double half_of(double v) {
+    return __hiloint2double(__double2hiint(v) - 0x00100000, __double2loint(v));
+}
+
 // Biased exponent of v (0 for zeros and subnormals, 2047 for inf/NaN).
 __device__ __forceinline__ unsigned div_exponent(double v) {
     return (static_cast<unsigned>(__double2hiint(v)) >> 20) & 0x7FFu;

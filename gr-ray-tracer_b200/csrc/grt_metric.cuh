@@ -129,8 +129,7 @@ GRT_DEV Rhs7 ks_rhs(double x, double y, double z, double pt, double px, double p
 }
 
 // ks_rhs with every quotient formed from the correctly rounded reciprocal of
-// its denominator (six of them: S, 2r, B, r, D, D^2; five reciprocal
-// evaluations, since RN(1/(2r)) = RN(1/r) / 2) by div_by, which rounds like an
+// its denominator (S, r, B, D, D^2, and 2r through r) by div_by, which rounds like an
 // IEEE division while no value under- or overflows.  That holds in
 // the box this checks: x, y, z each an exact zero or of magnitude in
 // [2^-20, 2^20], r in [2^-24, 2^20] and S in [2^-60, 2^42], with a spin of
@@ -141,7 +140,7 @@ GRT_DEV Rhs7 ks_rhs(double x, double y, double z, double pt, double px, double p
 // divided by at most r^8 <= 2^160.  Outside it, and where a denominator's low
 // word is all ones (once in 2^32: it covers the one significand that
 // rcp_rn_core does not round), `ok` is false and the caller evaluates ks_rhs.
-// The expression tree is ks_rhs's, so the result equals ks_rhs bit for bit.
+// Every rounding is one of ks_rhs's, so the result equals ks_rhs bit for bit.
 // The check comes last: nothing here traps, and without a branch in the middle
 // the right-hand side is one block for the compiler to schedule.  The upper
 // bounds of x, y and z are those of r (|z| <= r, x^2 + y^2 <= r^2 + a^2).
@@ -155,81 +154,90 @@ GRT_DEV double rhs_recip(double b) {
     else return div_recip(b);
 }
 
-template <bool BF>
-GRT_DEV double rhs_sqrt(double v) {
-    if constexpr (BF) return sqrt_rn_box(v);
-    else return sqrt(v);
-}
-
 GRT_DEV unsigned low_word(double v) { return static_cast<unsigned>(__double2loint(v)); }
 
+// The square root of v and the correctly rounded reciprocal of the root.
+template <bool BF>
+GRT_DEV double rhs_sqrt_recip(double v, double& recip) {
+    if constexpr (BF) {
+        double y;
+        const double s = sqrt_rn_box(v, y);
+        recip = rcp_rn_near(s, y);
+        return s;
+    } else {
+        const double s = sqrt(v);
+        recip = div_recip(s);
+        return s;
+    }
+}
+
+// ks_rhs's tree with its factors of two moved: a product with a power of two
+// rounds nothing, so x / (2 r) is half of x / r, 4 r^3 d is 2 r^3 (2 d), and a
+// factor left in front of a sum goes into one fma that rounds as the sum does
+// (fma(2, q, u) = RN(u + 2 q)).  d_k = 2 dr/dx^k stands for dr/dx^k, and
+// dH/dx^k is carried halved for k = 0, 1.
 template <bool BF = false>
 GRT_DEV Rhs7 ks_rhs_rcp(double x, double y, double z, double pt, double px, double py, double pz,
                         double a, double M, bool& ok) {
     const double rsq = x * x + y * y + z * z;
-    const double A = rsq - a * a;
+    const double aa = a * a;
+    const double A = rsq - aa;
+    const double az = a * z, az2 = az * az;
     // Two square-root sites (unlike ks_radius): the reciprocal of S and the
     // quotients that use it then overlap the second square root, which
     // measured 3% faster on a lane-per-SM workload than one rolled site.
-    const double S = rhs_sqrt<BF>(A * A + 4.0 * ((a * z) * (a * z)));
-    const double r = rhs_sqrt<BF>(0.5 * (A + S));
+    double yS, yr;
+    const double S = rhs_sqrt_recip<BF>(fma(4.0, az2, A * A), yS);
+    const double r = rhs_sqrt_recip<BF>(half_of(A + S), yr);
     Rhs7 o;
-    const double yS = rhs_recip<BF>(S);
     const double opas = 1.0 + div_by(A, S, yS);
-    const double two_r = 2.0 * r;
-    // RN(1/(2r)) = RN(1/r) / 2 exactly: r is inside the box, so no rounding
-    // step under- or overflows
-    const double yr = rhs_recip<BF>(r);
-    const double y2r = 0.5 * yr;
-    const double dr0 = div_by(x * opas, two_r, y2r);
-    const double dr1 = div_by(y * opas, two_r, y2r);
-    const double dr2 = div_by(z * opas + div_by(2.0 * (a * a) * z, S, yS), two_r, y2r);
-    const double B = r * r + a * a;
+    const double c2 = 2.0 * aa * z;
+    const double d0 = div_by(x * opas, r, yr);
+    const double d1 = div_by(y * opas, r, yr);
+    const double d2 = div_by(z * opas + div_by(c2, S, yS), r, yr);
+    const double r2 = r * r;
+    const double B = r2 + aa;
     const double yB = rhs_recip<BF>(B);
     const double l1 = div_by(r * x + a * y, B, yB);
     const double l2 = div_by(r * y - a * x, B, yB);
     const double l3 = div_by(z, r, yr);
-    const double dB0 = 2.0 * r * dr0;
-    const double dB1 = 2.0 * r * dr1;
-    const double dB2 = 2.0 * r * dr2;
-    const double dl01 = div_by((dr0 * x + r) - l1 * dB0, B, yB);
-    const double dl02 = div_by((dr0 * y - a) - l2 * dB0, B, yB);
-    const double dl03 = div_by(-(l3 * dr0), r, yr);
-    const double dl11 = div_by((dr1 * x + a) - l1 * dB1, B, yB);
-    const double dl12 = div_by((dr1 * y + r) - l2 * dB1, B, yB);
-    const double dl13 = div_by(-(l3 * dr1), r, yr);
-    const double dl21 = div_by(dr2 * x - l1 * dB2, B, yB);
-    const double dl22 = div_by(dr2 * y - l2 * dB2, B, yB);
-    const double dl23 = div_by(1.0 - l3 * dr2, r, yr);
-    const double r2 = r * r;
+    const double dB0 = r * d0;
+    const double dB1 = r * d1;
+    const double dB2 = r * d2;
+    const double dl01 = div_by(fma(0.5, d0 * x, r) - l1 * dB0, B, yB);
+    const double dl02 = div_by(fma(0.5, d0 * y, -a) - l2 * dB0, B, yB);
+    const double m03 = div_by(l3 * d0, r, yr);  // -2 dl03
+    const double dl11 = div_by(fma(0.5, d1 * x, a) - l1 * dB1, B, yB);
+    const double dl12 = div_by(fma(0.5, d1 * y, r) - l2 * dB1, B, yB);
+    const double m13 = div_by(l3 * d1, r, yr);  // -2 dl13
+    const double dl21 = div_by(fma(0.5, d2 * x, -(l1 * dB2)), B, yB);
+    const double dl22 = div_by(fma(0.5, d2 * y, -(l2 * dB2)), B, yB);
+    const double dl23 = div_by(fma(-0.5, l3 * d2, 1.0), r, yr);
     const double r3 = r2 * r;
-    const double D = r3 * r + (a * z) * (a * z);
+    const double D = r3 * r + az2;
     const double yD = rhs_recip<BF>(D);
     const double H = div_by(M * r3, D, yD);
-    const double four_r3 = 4.0 * r3;
-    const double dD0 = four_r3 * dr0;
-    const double dD1 = four_r3 * dr1;
-    const double dD2 = four_r3 * dr2 + 2.0 * (a * a) * z;
     const double three_r2 = 3.0 * r2;
     const double DD = D * D;
     const double yDD = rhs_recip<BF>(DD);
-    const double dH0 = div_by(M * (three_r2 * dr0 * D - r3 * dD0), DD, yDD);
-    const double dH1 = div_by(M * (three_r2 * dr1 * D - r3 * dD1), DD, yDD);
-    const double dH2 = div_by(M * (three_r2 * dr2 * D - r3 * dD2), DD, yDD);
+    // dD_k = 2 g_k, and 2 g_2 + 2 a^2 z for k = 2
+    const double g0 = r3 * d0, g1 = r3 * d1, g2 = r3 * d2;
+    const double h0 = div_by(M * fma(0.25, three_r2 * d0 * D, -(r3 * g0)), DD, yDD);  // dH0 / 2
+    const double h1 = div_by(M * fma(0.25, three_r2 * d1 * D, -(r3 * g1)), DD, yDD);
+    const double dH2 = div_by(M * fma(0.5, three_r2 * d2 * D, -(r3 * fma(2.0, g2, c2))), DD, yDD);
+    const double ldp = ((-pt + l1 * px) + l2 * py) + l3 * pz;
+    const double Hl = H * ldp;
+    o.t = fma(2.0, Hl, -pt);
+    o.x = fma(-2.0, H * l1 * ldp, px);
+    o.y = fma(-2.0, H * l2 * ldp, py);
+    o.z = fma(-2.0, H * l3 * ldp, pz);
+    const double ldp2 = ldp * ldp, two_ldp2 = 2.0 * ldp2;
+    o.px = fma(2.0, Hl * fma(-0.5, m03 * pz, dl01 * px + dl02 * py), h0 * two_ldp2);
+    o.py = fma(2.0, Hl * fma(-0.5, m13 * pz, dl11 * px + dl12 * py), h1 * two_ldp2);
+    o.pz = fma(2.0, Hl * ((dl21 * px + dl22 * py) + dl23 * pz), dH2 * ldp2);
     const unsigned small = div_min_nonzero(div_min_nonzero(div_min_nonzero(~0u, x), y), z);
     const unsigned ones = max(max(max(low_word(S), low_word(r)), max(low_word(B), low_word(D))), low_word(DD));
     ok = small >= ((1023u - 20u) << 20) - 1u && div_within<-24, 19>(r) && div_within<-60, 41>(S) && ones != ~0u;
-    const double ldp = ((-pt + l1 * px) + l2 * py) + l3 * pz;
-    const double twoH = 2.0 * H;
-    o.t = -pt - (-twoH) * ldp;
-    o.x = px - twoH * l1 * ldp;
-    o.y = py - twoH * l2 * ldp;
-    o.z = pz - twoH * l3 * ldp;
-    const double ldp2 = ldp * ldp;
-    const double twoHl = twoH * ldp;
-    o.px = dH0 * ldp2 + twoHl * ((dl01 * px + dl02 * py) + dl03 * pz);
-    o.py = dH1 * ldp2 + twoHl * ((dl11 * px + dl12 * py) + dl13 * pz);
-    o.pz = dH2 * ldp2 + twoHl * ((dl21 * px + dl22 * py) + dl23 * pz);
     return o;
 }
 

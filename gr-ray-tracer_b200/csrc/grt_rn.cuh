@@ -80,13 +80,29 @@ __device__ __forceinline__ double rcp_rn_box(double b) {
     return ones ? __hiloint2double(static_cast<int>(hi_ones), 1) : y;
 }
 
-__device__ __forceinline__ double sqrt_rn_box(double v) {
-    double y = rsqrt_seed(v);
+// y receives 1/sqrt(v) to within a rounding and 2^-58: a seed for the
+// reciprocal of the root (rcp_rn_near).
+__device__ __forceinline__ double sqrt_rn_box(double v, double& y) {
+    y = rsqrt_seed(v);
     const double e = fma(-(v * y), y, 1.0);
     y = fma(y * e, fma(0.375, e, 0.5), y);
     const double s = v * y;
     const double r = fma(-s, s, v);
     return fma(r, 0.5 * y, s);
+}
+
+__device__ __forceinline__ double sqrt_rn_box(double v) {
+    double y;
+    return sqrt_rn_box(v, y);
+}
+
+// RN(1/b), b's significand not all ones, from y within 2^-50 of it: the first
+// step squares that, which leaves the rounding alone, the second is Markstein's.
+__device__ __forceinline__ double rcp_rn_near(double b, double y) {
+    double e = fma(-b, y, 1.0);
+    y = fma(y, e, y);
+    e = fma(-b, y, 1.0);
+    return fma(y, e, y);
 }
 
 }  // namespace dev

@@ -229,7 +229,7 @@ GRT_DEV void rk4_step(double s[8], double dt, const KParams& kp, int fast) {
         for (int c = 0; c < 7; ++c) t[sidx(c)] = s[sidx(c)] + cdt * k.v[c];
         k = RHS::eval(t, kp, fast);
 #pragma unroll
-        for (int c = 0; c < 7; ++c) sum.v[c] = sum.v[c] + w * k.v[c];
+        for (int c = 0; c < 7; ++c) sum.v[c] = fma(w, k.v[c], sum.v[c]);  // w k is exact
         cdt = st == 2 ? dt : 0.5 * dt;
         w = st == 2 ? 1.0 : 2.0;
     }
