@@ -193,6 +193,7 @@ struct grt_ctx {
     DevBuf<int> group_chan_dev, chan_img_dev;
     DevBuf<unsigned long long> share_state;  // [geodesics] lead / finished channels (KParams::share_state)
     DevBuf<long long> calls_carry;           // [queue] calls taken in the backward-leg launch
+    DevBuf<unsigned> stragglers;             // [queue] rays handed on between launches (KParams::stragglers)
     // output-step archives: gathered fields on the device, then in pinned host memory
     DevBuf<unsigned char> out_stage;
     unsigned char* host_out = nullptr;
@@ -453,7 +454,8 @@ void grt_destroy(grt_ctx* c) {
     c->nckpt.release(); c->adj_overflow.release(); c->call0.release();
     c->adj_nfull.release(); c->adj_full.release();
     c->bimage.release(); c->bspectrum.release(); c->barrived.release();
-    c->share_state.release(); c->calls_carry.release(); c->out_stage.release();
+    c->share_state.release(); c->calls_carry.release(); c->stragglers.release();
+    c->out_stage.release();
     if (c->host_out) cudaFreeHost(c->host_out);
     if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
     if (c->graph) cudaGraphDestroy(c->graph);
@@ -1139,7 +1141,10 @@ bool split_legs(const grt_ctx* c) { return c->lc.split_legs != 0 && c->p.mode ==
 // Device buffers a trace needs besides the photons; allocated before any
 // launch or graph capture.
 grt_status prepare_trace_buffers(grt_ctx* c, unsigned long long queue) {
-    if (split_legs(c)) GRT_CUDA(c, c->calls_carry.alloc(queue), "alloc call carry");
+    if (split_legs(c)) {
+        GRT_CUDA(c, c->calls_carry.alloc(queue), "alloc call carry");
+        if (queue < (1ull << 32) && c->stragglers.alloc(queue) != cudaSuccess) cudaGetLastError();  // done without
+    }
     return GRT_OK;
 }
 
@@ -1189,17 +1194,36 @@ cudaError_t launch_trace(const grt_ctx* c, const grt::KParams& kp_in, size_t sme
         const int leg = p.mode == GRT_MODE_DISK && kp.ngroups == 0 ? 3 : 0;
         return grt::launch_trace(kp, mixed, leg, p.integrator, c->sm_count, bps, smem, c->stream);
     }
+    // With many tiles for every warp, a warp's last rays are handed on to a
+    // second launch of the leg.  With few, the rays handed on only finish later:
+    // trace ms without / with at 2.1 tiles for every warp 1.92 / 2.00, 3.5 2.83 /
+    // 2.86, 5.4 3.82 / 3.75, 8.4 6.01 / 5.84, 13 8.77 / 8.47.
+    const unsigned long long claims = kp.grab > 0 ? (kp.n + kp.grab - 1) / kp.grab : 0;
+    const bool hand_on = claims >= 5ull * 4 * bps * c->sm_count && kp.refill_threshold == 32 &&
+                         c->stragglers.count >= kp.n;
     cudaError_t e = cudaMemsetAsync(kp.calls_carry, 0, kp.n * sizeof(long long), c->stream);
-    if (e == cudaSuccess)
-        e = grt::launch_trace(kp, mixed, 1, p.integrator, c->sm_count, bps, smem, c->stream);
+    auto leg = [&](int which) {
+        grt::KParams k = kp;
+        if (hand_on) k.stragglers = c->stragglers.ptr;
+        if (e == cudaSuccess) e = grt::launch_trace(k, mixed, which, p.integrator, c->sm_count, bps, smem, c->stream);
+        if (!hand_on || e != cudaSuccess) return;
+        k.stragglers = nullptr;
+        k.order = c->stragglers.ptr;
+        k.n_dev = &kp.counters->handed_on;
+        k.resume = 1;
+        e = cudaMemsetAsync(&kp.counters->queue_head, 0, sizeof(unsigned long long), c->stream);
+        if (e == cudaSuccess) e = grt::launch_trace(k, mixed, which, p.integrator, c->sm_count, bps, smem, c->stream);
+        if (e == cudaSuccess)
+            e = cudaMemsetAsync(&kp.counters->handed_on, 0, sizeof(unsigned long long), c->stream);
+    };
+    leg(1);
     if (e == cudaSuccess)
         e = grt::launch_generate_pending(
             kp, c->sm_count,
             grt::dev_trace_smem_bytes(0, 128, c->fluid_available && c->separable, c->nr, c->nth, c->nph), c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(&kp.counters->queue_head, 0, sizeof(unsigned long long), c->stream);
     kp.sm_claims += grt::kSmClaimSlots;
-    if (e == cudaSuccess)
-        e = grt::launch_trace(kp, mixed, 2, p.integrator, c->sm_count, bps, smem, c->stream);
+    leg(2);
     return e;
 }
 

@@ -73,7 +73,7 @@ struct KCounters {
     unsigned long long calls;             // functor invocations on live photons
     unsigned long long max_term_step;     // largest global step index at which a photon terminated, +1
     unsigned long long timed_out;         // warps that hit their iteration limit
-    unsigned long long pad;
+    unsigned long long handed_on;         // stragglers put on KParams::stragglers
 };
 
 // One image of a launch: the camera plane of integrate_cart_ks.hpp:96-107
@@ -148,6 +148,15 @@ struct KParams {
     // image mode: queue position -> queue index, so that each warp's 32
     // claims are an 8 x 4 tile of one image's pixels (nullptr = identity)
     const unsigned* order;
+    // Stragglers (image-mode legs with more tiles than warps): a warp left with
+    // at most kStragglers live lanes while tiles remain puts their queue
+    // indices here (counted in KCounters::handed_on) and takes its next tile; a
+    // launch with resume = 1 over that list (order = stragglers, n_dev its
+    // count) then continues them, 32 to a warp.  nullptr: none
+    unsigned* stragglers;
+    const unsigned long long* n_dev;  // queue length on the device (nullptr: n)
+    int resume;
+    int pad_resume;
     int refill_threshold;      // idle lanes before a warp refills (1..32)
     int grab;                  // photons claimed per queue access (per warp)
     const double* m_abs;       // optional per-cell multipliers on dtau (nullptr = 1)

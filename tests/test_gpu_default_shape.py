@@ -1,7 +1,10 @@
 """The refill threshold the library picks while no launch shape is set (32 in
 image mode, 4 in disk mode) changes no photon: against the thresholds at the
 ends of the range, set by hand, with more rays than the resident lanes so that
-warps do refill."""
+warps do refill.  Images of more than five tiles for every resident warp also
+hand the last rays of a tile on to a second launch at a threshold of 32; two
+frequency channels that share their geodesics as well, and a run cut short by
+its step count."""
 
 import numpy as np
 import pytest
@@ -21,12 +24,20 @@ def photons(gpu, p, grid, start, **shape):
         return ctx.download_photons().as_dict(), stats
 
 
-@pytest.mark.parametrize("mode", ["image", "disk"])
+@pytest.mark.parametrize("mode", ["image", "image_large", "image_cut", "channels", "disk"])
 def test_default_refill_gives_the_same_photons(gpu, mode):
-    if mode == "image":
-        w = workloads.scaled(workloads.C2, pixels=293, grid=(32, 16, 16), image_nx=293, image_ny=293)
+    if mode != "disk":
+        px = 293 if mode == "image" else 651
+        w = workloads.scaled(workloads.C2, pixels=px, grid=(32, 16, 16), image_nx=px, image_ny=px,
+                             max_steps=27 if mode == "image_cut" else 4000,
+                             precision=abi.PREC_MIXED if mode == "channels" else abi.PREC_FP64)
         p, grid = w.params(), w.torus()
-        start = lambda ctx: ctx.init_image_photons(293, 293)  # noqa: E731
+        if mode == "channels":
+            specs = [abi.ImageSpec.from_params(p, px, px, custom_frequency_hz=f, emission_coefficient=f / 2.3e11)
+                     for f in (2.3e11, 8.6e10)]
+            start = lambda ctx: ctx.init_image_batch(specs)  # noqa: E731
+        else:
+            start = lambda ctx: ctx.init_image_photons(px, px)  # noqa: E731
     else:
         w = workloads.DiskWorkload("disk", (48, 24, 24), 0.9, 60.0)
         p, grid = w.params(), torus.benchmark_torus(*w.grid, spin=w.spin)
