@@ -322,8 +322,8 @@ cudaError_t launch_gather_fields(const GatherArgs& a, int sm_count, cudaStream_t
 }
 
 cudaError_t launch_trace(const KParams& kp, bool mixed, int leg, int integrator, int sm_count, int blocks_per_sm,
-                         size_t smem, cudaStream_t stream) {
-    const int blocks = sm_count * blocks_per_sm;
+                         int launched, size_t smem, cudaStream_t stream) {
+    const int blocks = sm_count * launched;
     switch (leg + (mixed ? 4 : 0)) {
         case 0: return launch_trace_fp64_leg0(kp, integrator, blocks_per_sm, blocks, smem, stream);
         case 1: return launch_trace_fp64_leg1(kp, integrator, blocks_per_sm, blocks, smem, stream);

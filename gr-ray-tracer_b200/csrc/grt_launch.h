@@ -241,9 +241,10 @@ cudaError_t launch_trace_mixed_leg3(const KParams& kp, int integrator, int block
 // (photons with calls_carry < 0), one thread per queue index; smem holds the
 // staged axes (dev_trace_smem_bytes with integrator 0).
 cudaError_t launch_generate_pending(const KParams& kp, int sm_count, size_t smem, cudaStream_t stream);
-// sm_count * blocks_per_sm blocks of the form's (FP64 or mixed) kernel for `leg`.
+// sm_count * launched blocks of the form's (FP64 or mixed) kernel for `leg`
+// compiled for blocks_per_sm (launched <= blocks_per_sm).
 cudaError_t launch_trace(const KParams& kp, bool mixed, int leg, int integrator, int sm_count, int blocks_per_sm,
-                         size_t smem, cudaStream_t stream);
+                         int launched, size_t smem, cudaStream_t stream);
 cudaError_t launch_init_image(const InitImageArgs& args, cudaStream_t stream);
 cudaError_t launch_screen_order(const ScreenOrderArgs& a, cudaStream_t stream);
 cudaError_t launch_init_disk(const DiskInitArgs& a, cudaStream_t stream);

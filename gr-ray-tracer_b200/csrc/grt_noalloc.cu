@@ -120,10 +120,12 @@ __global__ void __launch_bounds__(128, B) trace_noalloc(const __grid_constant__ 
 
 template <int INTEGRATOR, int B>
 cudaError_t launch_noalloc(const grt::KParams& kp, int sms, size_t smem, cudaStream_t stream) {
+    // with a claim quota, the blocks that hold the claims: one warp a scheduler first
+    const int per_sm = kp.sm_quota ? static_cast<int>((kp.sm_quota + 3) / 4) : B;
     cudaError_t e = cudaFuncSetAttribute(trace_noalloc<INTEGRATOR, B>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(smem));
     if (e != cudaSuccess) return e;
-    trace_noalloc<INTEGRATOR, B><<<sms * B, 128, smem, stream>>>(kp);
+    trace_noalloc<INTEGRATOR, B><<<sms * per_sm, 128, smem, stream>>>(kp);
     return cudaGetLastError();
 }
 
