@@ -223,7 +223,7 @@ struct grt_ctx {
     // upload and the products' copy-back run on copy_stream, the trace on
     // stream; one render in flight per context
     cudaStream_t copy_stream = nullptr;
-    cudaEvent_t ev_uploaded = nullptr, ev_traced = nullptr, ev_done = nullptr;
+    cudaEvent_t ev_uploaded = nullptr, ev_rest = nullptr, ev_traced = nullptr, ev_done = nullptr;
     bool render_pending = false;
 };
 
@@ -421,6 +421,7 @@ grt_status grt_create(const grt_params* p, grt_ctx** out) {
         cudaEventCreateWithFlags(&c->ev_part[2], cudaEventDisableTiming) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_uploaded, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_rest, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_traced, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_done, cudaEventDisableTiming) != cudaSuccess) {
         grt_destroy(c);
@@ -464,6 +465,7 @@ void grt_destroy(grt_ctx* c) {
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
     if (c->ev_uploaded) cudaEventDestroy(c->ev_uploaded);
+    if (c->ev_rest) cudaEventDestroy(c->ev_rest);
     if (c->ev_traced) cudaEventDestroy(c->ev_traced);
     if (c->ev_done) cudaEventDestroy(c->ev_done);
     if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
@@ -1186,8 +1188,11 @@ int set_claim_quota(const grt_ctx* c, grt::KParams& kp, int bps) {
 // the backward-leg launch, the packet generation of the rays it stopped at their
 // first fluid contact, and, with the queue head reset, the forward-leg launch
 // over the same queue.  `chunk` selects the chunk's claim counters, which the
-// caller has zeroed, as it has the launch counters (reset_trace).
-cudaError_t launch_trace(const grt_ctx* c, const grt::KParams& kp_in, size_t smem, bool split, int chunk = 0) {
+// caller has zeroed, as it has the launch counters (reset_trace).  With `rest`, the
+// launches that read or write a photon's id, frequency, emission-frame energy or
+// screen position wait for that event: all but the backward leg's.
+cudaError_t launch_trace(const grt_ctx* c, const grt::KParams& kp_in, size_t smem, bool split, int chunk = 0,
+                         cudaEvent_t rest = nullptr) {
     const int bps = trace_blocks_per_sm(c, kp_in.n);
     grt::KParams kp = kp_in;
     const int launched = set_claim_quota(c, kp, bps);
@@ -1197,6 +1202,10 @@ cudaError_t launch_trace(const grt_ctx* c, const grt::KParams& kp_in, size_t sme
     if (!split) {
         // disk mode: the whole-ray kernel without the image-mode code (leg 3)
         const int leg = p.mode == GRT_MODE_DISK && kp.ngroups == 0 ? 3 : 0;
+        if (rest) {
+            const cudaError_t ew = cudaStreamWaitEvent(c->stream, rest, 0);
+            if (ew != cudaSuccess) return ew;
+        }
         return grt::launch_trace(kp, mixed, leg, p.integrator, c->sm_count, bps, launched, smem, c->stream);
     }
     // With many tiles for every warp, a warp's last rays are handed on to a
@@ -1222,6 +1231,7 @@ cudaError_t launch_trace(const grt_ctx* c, const grt::KParams& kp_in, size_t sme
             e = cudaMemsetAsync(&kp.counters->handed_on, 0, sizeof(unsigned long long), c->stream);
     };
     leg(1);
+    if (e == cudaSuccess && rest) e = cudaStreamWaitEvent(c->stream, rest, 0);
     if (e == cudaSuccess)
         e = grt::launch_generate_pending(
             kp, c->sm_count,
@@ -1713,9 +1723,20 @@ static grt_status enqueue_render(grt_ctx* c, const grt_photon_soa* s, grt_image_
     kp.step0 = 0;
     kp.budget = c->p.max_steps;
     kp.max_iterations = iteration_limit(c, kp, n, c->sm_count * trace_blocks_per_sm(c, kp.n), 128);
-    GRT_CUDA(c, cudaMemcpyAsync(c->ph.block.ptr, s->id, grt_photon_block_bytes(n), cudaMemcpyHostToDevice,
-                                c->copy_stream), "H2D photons");
+    // What the backward leg reads or writes comes first (x0 .. dlambda, terminate,
+    // phase: 106 of a photon's 146 bytes), the rest under it.
+    const unsigned char* host = reinterpret_cast<const unsigned char*>(s->id);
+    auto fields = [&](int from, int to) {  // the fields [from, to) of the block
+        const size_t at = photon_field_offset(n, from);
+        const size_t end = to == 20 ? grt_photon_block_bytes(n) : photon_field_offset(n, to);
+        return cudaMemcpyAsync(c->ph.block.ptr + at, host + at, end - at, cudaMemcpyHostToDevice, c->copy_stream);
+    };
+    GRT_CUDA(c, fields(3, 16), "H2D photons");
+    GRT_CUDA(c, fields(18, 20), "H2D photons");
     GRT_CUDA(c, cudaEventRecord(c->ev_uploaded, c->copy_stream), "event");
+    GRT_CUDA(c, fields(0, 3), "H2D photons");
+    GRT_CUDA(c, fields(16, 18), "H2D photons");
+    GRT_CUDA(c, cudaEventRecord(c->ev_rest, c->copy_stream), "event");
     GRT_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_uploaded, 0), "stream wait");
     if (c->groups_share && c->geodesics)
         GRT_CUDA(c, cudaMemsetAsync(c->share_state.ptr, 0, c->geodesics * sizeof(unsigned long long), c->stream),
@@ -1726,7 +1747,7 @@ static grt_status enqueue_render(grt_ctx* c, const grt_photon_soa* s, grt_image_
              "count_terminated");
     GRT_CUDA(c, reset_trace(c), "memset counters");
     GRT_CUDA(c, cudaEventRecord(c->ev0, c->stream), "event");
-    const cudaError_t e = launch_trace(c, kp, trace_smem(c), split_legs(c));
+    const cudaError_t e = launch_trace(c, kp, trace_smem(c), split_legs(c), 0, c->ev_rest);
     if (e != cudaSuccess) return cuda_fail(c, e, "trace launch");
     GRT_CUDA(c, cudaEventRecord(c->ev1, c->stream), "event");
     grt_status st = launch_all_products(c);
