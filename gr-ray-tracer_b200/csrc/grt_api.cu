@@ -152,9 +152,8 @@ struct grt_ctx {
     grt::KCounters* host_counters = nullptr;  // pinned
     // products of grt_get_image_products, one block: [4][ny][nx], spectrum, arrived
     DevBuf<double> image;
-    double* host_products = nullptr;  // pinned stage of that block
-    size_t host_products_values = 0;
-    cudaEvent_t ev_part[3] = {nullptr, nullptr, nullptr};
+    unsigned char* host_stage = nullptr;  // pinned: two halves of kStagePiece bytes
+    cudaEvent_t ev_half[2] = {nullptr, nullptr};
     DevBuf<unsigned long long> scratch_u64;
     unsigned long long* host_u64 = nullptr;  // pinned
     grt_launch_config lc{128, 0, 8, 32, 1, 0, 0};
@@ -416,9 +415,8 @@ grt_status grt_create(const grt_params* p, grt_ctx** out) {
         cudaMallocHost(reinterpret_cast<void**>(&c->host_counters), kMaxChunks * sizeof(grt::KCounters)) != cudaSuccess ||
         cudaMallocHost(reinterpret_cast<void**>(&c->host_u64), 4 * sizeof(unsigned long long)) != cudaSuccess ||
         cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_part[0], cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_part[1], cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_part[2], cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_half[0], cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_half[1], cudaEventDisableTiming) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_uploaded, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_rest, cudaEventDisableTiming) != cudaSuccess ||
@@ -444,8 +442,8 @@ void grt_destroy(grt_ctx* c) {
     c->ph.release();
     c->counters.release();
     c->image.release(); c->scratch_u64.release();
-    if (c->host_products) cudaFreeHost(c->host_products);
-    for (cudaEvent_t e : c->ev_part)
+    if (c->host_stage) cudaFreeHost(c->host_stage);
+    for (cudaEvent_t e : c->ev_half)
         if (e) cudaEventDestroy(e);
     c->images_dev.release(); c->image_start_dev.release();
     c->group_qstart_dev.release(); c->group_chan_dev.release(); c->chan_img_dev.release();
@@ -1140,16 +1138,6 @@ unsigned long long iteration_limit(const grt_ctx* c, const grt::KParams& kp, uns
 // 2), unless the launch shape asks for one launch over whole rays.
 bool split_legs(const grt_ctx* c) { return c->lc.split_legs != 0 && c->p.mode == GRT_MODE_IMAGE; }
 
-// Device buffers a trace needs besides the photons; allocated before any
-// launch or graph capture.
-grt_status prepare_trace_buffers(grt_ctx* c, unsigned long long queue) {
-    if (split_legs(c)) {
-        GRT_CUDA(c, c->calls_carry.alloc(queue), "alloc call carry");
-        if (queue < (1ull << 32) && c->stragglers.alloc(queue) != cudaSuccess) cudaGetLastError();  // done without
-    }
-    return GRT_OK;
-}
-
 // Resident trace blocks per SM: the launch shape's, or with 0 (automatic)
 // in image mode the fewest of 2, 3, 4 that keep every geodesic of the queue
 // resident at once -- fewer blocks give each thread more registers (255, 170,
@@ -1167,6 +1155,28 @@ int trace_blocks_per_sm(const grt_ctx* c, unsigned long long queue) {
     for (int b = 2; b < 4; ++b)
         if (lanes * b >= queue) return b;
     return 4;
+}
+
+// Whether a split trace of `queue` rays hands a warp's last rays on to a second
+// launch of the leg (KParams::stragglers): with many tiles for every warp.
+// With few, the rays handed on only finish later: trace ms without / with at
+// 2.1 tiles for every warp 1.92 / 2.00, 3.5 2.83 / 2.86, 5.4 3.82 / 3.75, 8.4
+// 6.01 / 5.84, 13 8.77 / 8.47.
+bool hands_on(const grt_ctx* c, unsigned long long queue) {
+    const int refill = c->lc_set ? c->lc.refill_threshold : grt::default_refill(1);
+    const unsigned long long grab = static_cast<unsigned long long>(c->lc.photons_per_grab);
+    const unsigned long long warps = 4ull * c->sm_count * trace_blocks_per_sm(c, queue);
+    return refill == 32 && queue < (1ull << 32) && (queue + grab - 1) / grab >= 5 * warps;
+}
+
+// Device buffers a trace needs besides the photons; allocated before any
+// launch or graph capture.
+grt_status prepare_trace_buffers(grt_ctx* c, unsigned long long queue) {
+    if (split_legs(c)) {
+        GRT_CUDA(c, c->calls_carry.alloc(queue), "alloc call carry");
+        if (hands_on(c, queue) && c->stragglers.alloc(queue) != cudaSuccess) cudaGetLastError();  // done without
+    }
+    return GRT_OK;
 }
 
 // When every queue claim of a launch fits in its resident warps (C1, C2: no
@@ -1208,13 +1218,7 @@ cudaError_t launch_trace(const grt_ctx* c, const grt::KParams& kp_in, size_t sme
         }
         return grt::launch_trace(kp, mixed, leg, p.integrator, c->sm_count, bps, launched, smem, c->stream);
     }
-    // With many tiles for every warp, a warp's last rays are handed on to a
-    // second launch of the leg.  With few, the rays handed on only finish later:
-    // trace ms without / with at 2.1 tiles for every warp 1.92 / 2.00, 3.5 2.83 /
-    // 2.86, 5.4 3.82 / 3.75, 8.4 6.01 / 5.84, 13 8.77 / 8.47.
-    const unsigned long long claims = kp.grab > 0 ? (kp.n + kp.grab - 1) / kp.grab : 0;
-    const bool hand_on = claims >= 5ull * 4 * bps * c->sm_count && kp.refill_threshold == 32 &&
-                         c->stragglers.count >= kp.n;
+    const bool hand_on = hands_on(c, kp.n) && c->stragglers.count >= kp.n;
     cudaError_t e = cudaMemsetAsync(kp.calls_carry, 0, kp.n * sizeof(long long), c->stream);
     auto leg = [&](int which) {
         grt::KParams k = kp;
@@ -2010,54 +2014,66 @@ grt_status grt_adjoint_image_I(grt_ctx* c, const double* dL_dI, double* g_abs, d
 
 // The device block of launch_products to the caller's arrays.  Copies into
 // ordinary (pageable) memory go through a driver stage one by one, each waiting
-// for the last; through the context's pinned stage the block comes back in one
-// copy, or in four when it is large, so that the host copies one plane while
-// the next arrives.  Products of a 16 x 16 image 106 to 79 us, of 256 x 256
-// 260 to 197, of 509 x 283 451 to 369.
+// for the last; through the context's own pinned stage the block comes back in
+// pieces, one copied on by the host while the next arrives.  The stage is small
+// because pinning is slow: a stage of the whole block made the first products
+// of a context 3 ms slower at 256 x 256.  Products of a 16 x 16 image 106 to
+// 42 us, of 256 x 256 260 to 195, of 509 x 283 451 to 357 (pieces of 64, 128, 256
+// KiB: 314, 245, 210 at 256 x 256).
+constexpr size_t kStagePiece = 512u << 10;
 static grt_status copy_products_out(grt_ctx* c, size_t npix, size_t bins, grt_image_products* out) {
-    constexpr size_t kStageMost = 64u << 20, kOnePiece = 256u << 10;
-    const size_t values = 4 * npix + bins + 1;
-    double* dst[4] = {out->image_I, out->image_Q, out->image_U, out->image_V};
     cudaPointerAttributes at;
     const bool pageable = cudaPointerGetAttributes(&at, out->image_I) != cudaSuccess ||
                           at.type == cudaMemoryTypeUnregistered;
     cudaGetLastError();
-    if (!pageable || values * sizeof(double) > kStageMost) {
-        for (int q = 0; q < 4; ++q)
-            GRT_CUDA(c, cudaMemcpyAsync(dst[q], c->image.ptr + q * npix, npix * sizeof(double), cudaMemcpyDeviceToHost,
-                                        c->stream), "D2H image");
-        GRT_CUDA(c, cudaMemcpyAsync(out->spectrum_I, c->image.ptr + 4 * npix, bins * sizeof(double),
-                                    cudaMemcpyDeviceToHost, c->stream), "D2H spectrum");
-        GRT_CUDA(c, cudaMemcpyAsync(out->arrived_count, c->image.ptr + 4 * npix + bins, sizeof(uint64_t),
-                                    cudaMemcpyDeviceToHost, c->stream), "D2H arrived");
+    struct Part {
+        void* dst;
+        size_t bytes;
+    };
+    const Part parts[6] = {{out->image_I, npix * sizeof(double)}, {out->image_Q, npix * sizeof(double)},
+                           {out->image_U, npix * sizeof(double)}, {out->image_V, npix * sizeof(double)},
+                           {out->spectrum_I, bins * sizeof(double)}, {out->arrived_count, sizeof(uint64_t)}};
+    const unsigned char* src = reinterpret_cast<const unsigned char*>(c->image.ptr);
+    if (!pageable) {
+        for (const Part& part : parts) {
+            if (part.bytes)
+                GRT_CUDA(c, cudaMemcpyAsync(part.dst, src, part.bytes, cudaMemcpyDeviceToHost, c->stream), "D2H products");
+            src += part.bytes;
+        }
         fill_spectrum_frequencies(c->p, out->spectrum_frequency_hz);
         GRT_CUDA(c, cudaStreamSynchronize(c->stream), "products");
         return GRT_OK;
     }
-    if (c->host_products_values < values) {
-        if (c->host_products) cudaFreeHost(c->host_products);
-        c->host_products = nullptr;
-        c->host_products_values = 0;
-        GRT_CUDA(c, cudaMallocHost(reinterpret_cast<void**>(&c->host_products), values * sizeof(double)),
-                 "alloc products stage");
-        c->host_products_values = values;
-    }
-    double* h = c->host_products;
-    const int pieces = values * sizeof(double) > kOnePiece ? 4 : 1;
-    for (int q = 0; q < pieces; ++q) {
-        const size_t from = q * npix, to = q == pieces - 1 ? values : (q + 1) * npix;
-        GRT_CUDA(c, cudaMemcpyAsync(h + from, c->image.ptr + from, (to - from) * sizeof(double),
-                                    cudaMemcpyDeviceToHost, c->stream), "D2H products");
-        if (q < pieces - 1) GRT_CUDA(c, cudaEventRecord(c->ev_part[q], c->stream), "event");
-    }
+    if (!c->host_stage)
+        GRT_CUDA(c, cudaMallocHost(reinterpret_cast<void**>(&c->host_stage), 2 * kStagePiece), "alloc products stage");
+    const size_t total = (4 * npix + bins + 1) * sizeof(double);
+    const size_t pieces = (total + kStagePiece - 1) / kStagePiece;
+    auto fetch = [&](size_t k) {
+        const size_t from = k * kStagePiece, bytes = std::min(kStagePiece, total - from);
+        const cudaError_t e = cudaMemcpyAsync(c->host_stage + (k & 1) * kStagePiece, src + from, bytes,
+                                              cudaMemcpyDeviceToHost, c->stream);
+        return e == cudaSuccess ? cudaEventRecord(c->ev_half[k & 1], c->stream) : e;
+    };
+    for (size_t k = 0; k < pieces && k < 2; ++k) GRT_CUDA(c, fetch(k), "D2H products");
     fill_spectrum_frequencies(c->p, out->spectrum_frequency_hz);
-    for (int q = 0; q < 4; ++q) {
-        if (q < pieces - 1) GRT_CUDA(c, cudaEventSynchronize(c->ev_part[q]), "products");
-        else if (q == pieces - 1) GRT_CUDA(c, cudaStreamSynchronize(c->stream), "products");
-        std::memcpy(dst[q], h + q * npix, npix * sizeof(double));
+    int part = 0;
+    size_t done = 0;  // bytes of parts[part] written
+    for (size_t k = 0; k < pieces; ++k) {
+        GRT_CUDA(c, cudaEventSynchronize(c->ev_half[k & 1]), "products");
+        const unsigned char* h = c->host_stage + (k & 1) * kStagePiece;
+        for (size_t left = std::min(kStagePiece, total - k * kStagePiece); left > 0;) {
+            const size_t now = std::min(left, parts[part].bytes - done);
+            std::memcpy(static_cast<unsigned char*>(parts[part].dst) + done, h, now);
+            h += now;
+            left -= now;
+            done += now;
+            if (done == parts[part].bytes) {
+                ++part;
+                done = 0;
+            }
+        }
+        if (k + 2 < pieces) GRT_CUDA(c, fetch(k + 2), "D2H products");
     }
-    std::memcpy(out->spectrum_I, h + 4 * npix, bins * sizeof(double));
-    std::memcpy(out->arrived_count, h + 4 * npix + bins, sizeof(uint64_t));
     return GRT_OK;
 }
 
