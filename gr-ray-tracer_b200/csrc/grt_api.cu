@@ -152,8 +152,8 @@ struct grt_ctx {
     grt::KCounters* host_counters = nullptr;  // pinned
     // products of grt_get_image_products, one block: [4][ny][nx], spectrum, arrived
     DevBuf<double> image;
-    unsigned char* host_stage = nullptr;  // pinned: two halves of kStagePiece bytes
-    cudaEvent_t ev_half[2] = {nullptr, nullptr};
+    unsigned char* host_stage = nullptr;  // pinned, host_stage_bytes, at most kStageMax
+    size_t host_stage_bytes = 0;
     DevBuf<unsigned long long> scratch_u64;
     unsigned long long* host_u64 = nullptr;  // pinned
     grt_launch_config lc{128, 0, 8, 32, 1, 0, 0};
@@ -415,8 +415,6 @@ grt_status grt_create(const grt_params* p, grt_ctx** out) {
         cudaMallocHost(reinterpret_cast<void**>(&c->host_counters), kMaxChunks * sizeof(grt::KCounters)) != cudaSuccess ||
         cudaMallocHost(reinterpret_cast<void**>(&c->host_u64), 4 * sizeof(unsigned long long)) != cudaSuccess ||
         cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_half[0], cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_half[1], cudaEventDisableTiming) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_uploaded, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_rest, cudaEventDisableTiming) != cudaSuccess ||
@@ -443,8 +441,6 @@ void grt_destroy(grt_ctx* c) {
     c->counters.release();
     c->image.release(); c->scratch_u64.release();
     if (c->host_stage) cudaFreeHost(c->host_stage);
-    for (cudaEvent_t e : c->ev_half)
-        if (e) cudaEventDestroy(e);
     c->images_dev.release(); c->image_start_dev.release();
     c->group_qstart_dev.release(); c->group_chan_dev.release(); c->chan_img_dev.release();
     c->order_ph.release(); c->order_geo.release(); c->sm_claims.release(); c->screen_scratch.release();
@@ -2014,13 +2010,14 @@ grt_status grt_adjoint_image_I(grt_ctx* c, const double* dL_dI, double* g_abs, d
 
 // The device block of launch_products to the caller's arrays.  Copies into
 // ordinary (pageable) memory go through a driver stage one by one, each waiting
-// for the last; through the context's own pinned stage the block comes back in
-// pieces, one copied on by the host while the next arrives.  The stage is small
-// because pinning is slow: a stage of the whole block made the first products
-// of a context 3 ms slower at 256 x 256.  Products of a 16 x 16 image 106 to
-// 42 us, of 256 x 256 260 to 195, of 509 x 283 451 to 357 (pieces of 64, 128, 256
-// KiB: 314, 245, 210 at 256 x 256).
-constexpr size_t kStagePiece = 512u << 10;
+// for the last.  A small block comes back whole instead, in one copy into the
+// context's own pinned stage, and the host hands it out.  Products of a 16 x
+// 16 image 106 to 42 us.  The line is drawn by the cost of pinning, which the
+// first frame of a context pays.  At the 0.53 MB of a 128 x 128 image that
+// frame takes 1.0 ms more than a repeated one, with direct copies 0.9; at 16 x
+// 16 0.14 ms against 0.11.  A stage of 1 MiB in two pieces took 64 us off a 256
+// x 256 image's 260, and added 2 to 7 ms to a context's first frame at any size.
+constexpr size_t kStageMax = 640u << 10;
 static grt_status copy_products_out(grt_ctx* c, size_t npix, size_t bins, grt_image_products* out) {
     cudaPointerAttributes at;
     const bool pageable = cudaPointerGetAttributes(&at, out->image_I) != cudaSuccess ||
@@ -2034,45 +2031,30 @@ static grt_status copy_products_out(grt_ctx* c, size_t npix, size_t bins, grt_im
                            {out->image_U, npix * sizeof(double)}, {out->image_V, npix * sizeof(double)},
                            {out->spectrum_I, bins * sizeof(double)}, {out->arrived_count, sizeof(uint64_t)}};
     const unsigned char* src = reinterpret_cast<const unsigned char*>(c->image.ptr);
-    if (!pageable) {
+    const size_t total = (4 * npix + bins + 1) * sizeof(double);
+    fill_spectrum_frequencies(c->p, out->spectrum_frequency_hz);
+    if (!pageable || total > kStageMax) {
         for (const Part& part : parts) {
             if (part.bytes)
                 GRT_CUDA(c, cudaMemcpyAsync(part.dst, src, part.bytes, cudaMemcpyDeviceToHost, c->stream), "D2H products");
             src += part.bytes;
         }
-        fill_spectrum_frequencies(c->p, out->spectrum_frequency_hz);
         GRT_CUDA(c, cudaStreamSynchronize(c->stream), "products");
         return GRT_OK;
     }
-    if (!c->host_stage)
-        GRT_CUDA(c, cudaMallocHost(reinterpret_cast<void**>(&c->host_stage), 2 * kStagePiece), "alloc products stage");
-    const size_t total = (4 * npix + bins + 1) * sizeof(double);
-    const size_t pieces = (total + kStagePiece - 1) / kStagePiece;
-    auto fetch = [&](size_t k) {
-        const size_t from = k * kStagePiece, bytes = std::min(kStagePiece, total - from);
-        const cudaError_t e = cudaMemcpyAsync(c->host_stage + (k & 1) * kStagePiece, src + from, bytes,
-                                              cudaMemcpyDeviceToHost, c->stream);
-        return e == cudaSuccess ? cudaEventRecord(c->ev_half[k & 1], c->stream) : e;
-    };
-    for (size_t k = 0; k < pieces && k < 2; ++k) GRT_CUDA(c, fetch(k), "D2H products");
-    fill_spectrum_frequencies(c->p, out->spectrum_frequency_hz);
-    int part = 0;
-    size_t done = 0;  // bytes of parts[part] written
-    for (size_t k = 0; k < pieces; ++k) {
-        GRT_CUDA(c, cudaEventSynchronize(c->ev_half[k & 1]), "products");
-        const unsigned char* h = c->host_stage + (k & 1) * kStagePiece;
-        for (size_t left = std::min(kStagePiece, total - k * kStagePiece); left > 0;) {
-            const size_t now = std::min(left, parts[part].bytes - done);
-            std::memcpy(static_cast<unsigned char*>(parts[part].dst) + done, h, now);
-            h += now;
-            left -= now;
-            done += now;
-            if (done == parts[part].bytes) {
-                ++part;
-                done = 0;
-            }
-        }
-        if (k + 2 < pieces) GRT_CUDA(c, fetch(k + 2), "D2H products");
+    if (c->host_stage_bytes < total) {
+        if (c->host_stage) cudaFreeHost(c->host_stage);
+        c->host_stage = nullptr;
+        c->host_stage_bytes = 0;
+        GRT_CUDA(c, cudaMallocHost(reinterpret_cast<void**>(&c->host_stage), total), "alloc products stage");
+        c->host_stage_bytes = total;
+    }
+    GRT_CUDA(c, cudaMemcpyAsync(c->host_stage, src, total, cudaMemcpyDeviceToHost, c->stream), "D2H products");
+    GRT_CUDA(c, cudaStreamSynchronize(c->stream), "products");
+    const unsigned char* h = c->host_stage;
+    for (const Part& part : parts) {
+        if (part.bytes) std::memcpy(part.dst, h, part.bytes);
+        h += part.bytes;
     }
     return GRT_OK;
 }

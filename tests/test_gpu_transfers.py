@@ -1,6 +1,6 @@
 """Products and gradients by the different ways they leave the device: the image
-products through the pinned stage in one piece or several, or straight into
-page-locked arrays, against the products block of the same photons; the
+products through the pinned stage, straight into ordinary arrays or into
+page-locked ones, against the products block of the same photons; the
 differentiable render on device tensors against host arrays."""
 
 import numpy as np
@@ -11,9 +11,9 @@ from grt import abi, torus, workloads
 pytestmark = pytest.mark.gpu
 
 
-# 4 nx ny + bins + 1 values around one and two pieces of 512 KiB, and the ends of planes inside a piece
-@pytest.mark.parametrize("nx,ny,bins", [(1, 1, 1), (1, 3, 2), (37, 19, 128), (91, 90, 7), (128, 64, 1), (128, 64, 128), (128, 128, 1), (181, 181, 3),
-                                        (131, 77, 5), (300, 211, 64)])
+# 4 nx ny + bins + 1 values: the smallest, odd planes, the largest block of the stage (81,920) and one more, larger ones
+@pytest.mark.parametrize("nx,ny,bins", [(1, 1, 1), (1, 3, 2), (37, 19, 128), (91, 90, 7), (128, 64, 1), (128, 64, 128), (128, 128, 1), (143, 143, 123), (143, 143, 124),
+                                        (181, 181, 3), (131, 77, 5), (300, 211, 64)])
 def test_image_products_by_every_way_out(gpu, nx, ny, bins):
     import torch
     w = workloads.scaled(workloads.C2, pixels=nx, grid=(24, 16, 16), image_nx=nx, image_ny=ny, spectrum_bins=bins,
