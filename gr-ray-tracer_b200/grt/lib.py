@@ -203,6 +203,7 @@ class Context:
         self._h = C.c_void_p()
         self.params = params.copy()
         self._specs = []
+        self._cells = 0  # of the grid; buffers per cell must hold as many values
         rc = self.lib.grt_create(C.byref(self.params), C.byref(self._h))
         if rc != GRT_OK:
             raise GrtError(rc, "grt_create failed (needs an sm_100 device and valid params)")
@@ -245,15 +246,24 @@ class Context:
     def upload_grid(self, grid: dict | None):
         """grid: dict of the seven .npy arrays (name -> ndarray), or None for no fluid."""
         if grid is None:
+            self._cells = 0
             self._check(self.lib.grt_upload_grid(self._h, 0, 0, 0, *([None] * 7)))
             return
         keys = ("r.npy", "theta.npy", "phi.npy", "rho.npy", "Tgas.npy", "vel.npy", "mag.npy")
         arrs = [np.ascontiguousarray(grid[k], dtype=np.float64) for k in keys]
         nr, nth, nph = arrs[0].shape
+        self._cells = arrs[0].size
         self._check(self.lib.grt_upload_grid(self._h, nr, nth, nph, *[_dp(a) for a in arrs]))
 
     def upload_grid_numpy_dir(self, path):
         self._check(self.lib.grt_upload_grid_numpy_dir(self._h, str(path).encode()))
+        self._cells = np.load(Path(path) / "r.npy", mmap_mode="r").size
+
+    def _check_cells(self, *buffers):
+        """The library reads or writes a value per cell of each buffer (arrays, device tensors, None)."""
+        for b in buffers:
+            if b is not None and (b.numel() if _on_device(b) else b.size) < self._cells:
+                raise ValueError(f"a buffer is too short for the grid's {self._cells} cells")
 
     def upload_photons(self, ph: PhotonArrays):
         soa = ph.soa()
@@ -342,6 +352,7 @@ class Context:
         contiguous float64 CUDA tensors that are complete; None = 1)."""
         self._mult = [m if m is None or _on_device(m) else np.ascontiguousarray(m, dtype=np.float64).ravel()
                       for m in (m_abs, m_emis)]
+        self._check_cells(*self._mult)
         self._check(self.lib.grt_set_cell_multipliers(self._h, *[_dp(m) if m is not None else None
                                                                   for m in self._mult]))
 
@@ -357,6 +368,7 @@ class Context:
             raise ValueError(f"dL/dimage_I must have shape {(self.params.image_ny, self.params.image_nx)}")
         ga = np.zeros(int(np.prod(grid_shape)))
         ge = np.zeros(int(np.prod(grid_shape)))
+        self._check_cells(ga, ge)
         self._check(self.lib.grt_adjoint_image_I(self._h, _dp(g), _dp(ga), _dp(ge)))
         return ga.reshape(grid_shape), ge.reshape(grid_shape)
 
@@ -367,6 +379,7 @@ class Context:
             raise ValueError(f"dL/dimage_I must have shape {(self.params.image_ny, self.params.image_nx)}")
         if not all(_on_device(t) for t in (dL_dimage_I, g_abs, g_emis)):
             raise TypeError("adjoint_image_I_device takes device tensors")
+        self._check_cells(g_abs, g_emis)
         self._check(self.lib.grt_adjoint_image_I(self._h, _dp(dL_dimage_I), _dp(g_abs), _dp(g_emis)))
 
     def run(self) -> dict:

@@ -1,0 +1,95 @@
+"""Host code of the C ABI where a call fails or a buffer does not fit, without a
+GPU: csrc/grt_api.cu and grt_host.cpp compiled against stand-ins for the CUDA
+runtime and the kernel launches (fake_cuda/fake_cuda.cpp)."""
+
+import ctypes as C
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+from grt import abi, lib, torus, workloads
+
+HERE = Path(__file__).resolve().parent
+SRC = HERE.parent / "gr-ray-tracer_b200" / "csrc"
+GRID = (8, 6, 5)
+
+
+@pytest.fixture(scope="module")
+def built(tmp_path_factory):
+    out = tmp_path_factory.mktemp("fake") / "libgrt_fake.so"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-w", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-I/usr/local/cuda/include",
+                    f"-I{SRC}", f"-I{HERE.parent / 'include'}", "-x", "c++", str(SRC / "grt_api.cu"),
+                    str(SRC / "grt_host.cpp"), str(HERE / "fake_cuda" / "fake_cuda.cpp"), "-o", str(out)], check=True)
+    return out
+
+
+@pytest.fixture
+def fake(built, monkeypatch):
+    monkeypatch.setattr(lib, "_lib", None)
+    L = lib.load(built)
+    L.fake_reset.argtypes = L.fake_limit.argtypes = L.fake_malloc.argtypes = [C.c_size_t]
+    L.fake_used.restype = C.c_size_t
+    L.fake_malloc.restype = C.c_void_p
+    L.fake_launches.restype = C.c_char_p
+    L.fake_reset(1 << 34)
+    yield L
+    assert L.fake_bad_accesses() == 0
+
+
+def image(px, **kw):
+    return workloads.scaled(workloads.C2, pixels=px, grid=GRID, image_nx=px, image_ny=px).params().update(**kw)
+
+
+def fluid():
+    return torus.benchmark_torus(*GRID, spin=workloads.C2.spin)
+
+
+def launches(fake, what=""):
+    return [line for line in fake.fake_launches().decode().splitlines() if line.startswith(what)]
+
+
+class DeviceArray:
+    """What Context asks of a CUDA tensor: a contiguous float64 one of the given shape."""
+    is_cuda, dtype = True, "torch.float64"
+
+    def __init__(self, fake, *shape):
+        self.shape = shape
+        self._ptr = fake.fake_malloc(8 * self.numel())
+
+    def is_contiguous(self):
+        return True
+
+    def numel(self):
+        return int(np.prod(self.shape))
+
+    def data_ptr(self):
+        return self._ptr
+
+
+@pytest.mark.parametrize("directory", [False, True])
+def test_buffers_shorter_than_the_grid_are_refused(fake, tmp_path, directory):
+    p, grid, cells = image(4), fluid(), int(np.prod(GRID))
+    with lib.Context(p) as ctx:
+        if directory:
+            for k in torus.FIELD_FILES:
+                np.save(tmp_path / k, grid[k])
+            ctx.upload_grid_numpy_dir(tmp_path)
+        else:
+            ctx.upload_grid(grid)
+        whole, short = DeviceArray(fake, *GRID), DeviceArray(fake, cells - 1)
+        for pair in ((short, None), (None, short), (whole, short), (np.ones(cells - 1), None), (np.ones(()), None)):
+            with pytest.raises(ValueError, match="cells"):
+                ctx.set_cell_multipliers(*pair)
+        ctx.set_cell_multipliers(whole, np.ones(GRID))
+        ctx.init_image_forward_photons(4, 4, 60.0)
+        ctx.forward_checkpointed(8)
+        dL = DeviceArray(fake, 4, 4)
+        for pair in ((short, whole), (whole, short)):
+            with pytest.raises(ValueError, match="cells"):
+                ctx.adjoint_image_I_device(dL, *pair)
+        with pytest.raises(ValueError, match="cells"):
+            ctx.adjoint_image_I(np.zeros((4, 4)), (cells - 1,))
+        ctx.adjoint_image_I_device(dL, whole, DeviceArray(fake, cells))
+        assert ctx.adjoint_image_I(np.zeros((4, 4)), GRID)[0].shape == GRID
