@@ -682,6 +682,28 @@ grt_status grt_upload_grid_numpy_dir(grt_ctx* c, const char* dir) {
                            a[5].data(), a[6].data());
 }
 
+// Leaves the context without photons and images.  An initialisation that fails
+// half-way does this: the counts, image tables and queue orders of the set
+// before it do not fit the buffers any more.  (Queue orders are used with
+// images only, and those kept are those of order_layout.)
+static void drop_photons(grt_ctx* c) {
+    ++c->generation;
+    c->n = 0;
+    c->initial_terminated = 0;
+    c->images.clear();
+    c->image_start.clear();
+    c->ngroups = 0;
+    c->groups_share = c->batched = c->have_images = false;
+    c->bproducts_valid = c->adj_ready = false;
+}
+
+// Room for n photons, or none at all.
+static cudaError_t alloc_photons(grt_ctx* c, size_t n) {
+    const cudaError_t e = c->ph.alloc(n);
+    if (e != cudaSuccess) drop_photons(c);
+    return e;
+}
+
 static grt_status count_initial_terminated(grt_ctx* c) {
     GRT_CUDA(c, cudaMemsetAsync(c->scratch_u64.ptr, 0, sizeof(unsigned long long), c->stream), "memset");
     GRT_CUDA(c, grt::launch_count_terminated(c->ph.term.ptr, c->n, c->scratch_u64.ptr, c->sm_count, c->stream),
@@ -699,7 +721,7 @@ grt_status grt_upload_photons(grt_ctx* c, const grt_photon_soa* s, size_t n) {
     if (n > (1ull << 40)) return fail(c, GRT_EINVAL, "photon count too large");
     const bool keep_images = c->have_images && n == c->n;  // same slots: photons keep their images
     c->adj_ready = false;
-    GRT_CUDA(c, c->ph.alloc(n), "alloc photons");
+    GRT_CUDA(c, alloc_photons(c, n), "alloc photons");
     c->n = n;
     c->bproducts_valid = false;
     if (!keep_images) {
@@ -932,24 +954,11 @@ grt_status set_screen_order(grt_ctx* c) {
     return GRT_OK;
 }
 
-grt_status set_image_set(grt_ctx* c, const grt_image_spec* specs, size_t nimages, uint64_t id_offset, bool batched,
-                         double forward_back = 0.0, uint64_t row0 = 0, uint64_t nrows = 0,
-                         bool random_screen = false) {
-    unsigned long long total = 0;
-    std::vector<unsigned long long> start(nimages + 1, 0);
-    for (size_t k = 0; k < nimages; ++k) {
-        const grt_image_spec& sp = specs[k];
-        if (sp.nx == 0 || sp.ny == 0 || sp.nx > (1u << 20) || sp.ny > (1u << 20))
-            return fail(c, GRT_EINVAL, "image " + std::to_string(k) + ": nx and ny must be in [1, 2^20]");
-        if (!(sp.camera_distance > 0.0) || !(sp.camera_width > 0.0) || !(sp.camera_height > 0.0) ||
-            !std::isfinite(sp.camera_theta) || !std::isfinite(sp.camera_phi))
-            return fail(c, GRT_EINVAL, "image " + std::to_string(k) +
-                                           ": camera distance, width and height must be positive and angles finite");
-        start[k] = total;
-        total += sp.nx * (nrows ? nrows : sp.ny);
-        if (total > (1ull << 40)) return fail(c, GRT_EINVAL, "photon count too large");
-    }
-    start[nimages] = total;
+// The image set of set_image_set, checked: start[k] is image k's first photon slot.
+grt_status lay_out_images(grt_ctx* c, const grt_image_spec* specs, size_t nimages,
+                          const std::vector<unsigned long long>& start, uint64_t id_offset, bool batched,
+                          double forward_back, uint64_t row0, uint64_t nrows, bool random_screen) {
+    const unsigned long long total = start[nimages];
     GRT_CUDA(c, c->ph.alloc(total), "alloc photons");
     ++c->generation;
     c->n = total;
@@ -1029,6 +1038,30 @@ grt_status set_image_set(grt_ctx* c, const grt_image_spec* specs, size_t nimages
     }
     const grt_status is = launch_image_inits(c);
     return is == GRT_OK && random_screen ? set_screen_order(c) : is;
+}
+
+grt_status set_image_set(grt_ctx* c, const grt_image_spec* specs, size_t nimages, uint64_t id_offset, bool batched,
+                         double forward_back = 0.0, uint64_t row0 = 0, uint64_t nrows = 0,
+                         bool random_screen = false) {
+    unsigned long long total = 0;
+    std::vector<unsigned long long> start(nimages + 1, 0);
+    for (size_t k = 0; k < nimages; ++k) {
+        const grt_image_spec& sp = specs[k];
+        if (sp.nx == 0 || sp.ny == 0 || sp.nx > (1u << 20) || sp.ny > (1u << 20))
+            return fail(c, GRT_EINVAL, "image " + std::to_string(k) + ": nx and ny must be in [1, 2^20]");
+        if (!(sp.camera_distance > 0.0) || !(sp.camera_width > 0.0) || !(sp.camera_height > 0.0) ||
+            !std::isfinite(sp.camera_theta) || !std::isfinite(sp.camera_phi))
+            return fail(c, GRT_EINVAL, "image " + std::to_string(k) +
+                                           ": camera distance, width and height must be positive and angles finite");
+        start[k] = total;
+        total += sp.nx * (nrows ? nrows : sp.ny);
+        if (total > (1ull << 40)) return fail(c, GRT_EINVAL, "photon count too large");
+    }
+    start[nimages] = total;
+    const grt_status st = lay_out_images(c, specs, nimages, start, id_offset, batched, forward_back, row0, nrows,
+                                         random_screen);
+    if (st != GRT_OK) drop_photons(c);
+    return st;
 }
 
 // Launch-wide part of a build_observation_products (observation.hpp:31-84) launch.
@@ -1336,18 +1369,11 @@ grt_status grt_init_disk_photons(grt_ctx* c, uint64_t id_offset, uint64_t* n_pho
     }
     off[ncell] = total;
     if (total > (1ull << 36)) return fail(c, GRT_EINVAL, "disk packet count too large: " + std::to_string(total));
-    GRT_CUDA(c, c->ph.alloc(total), "alloc photons");
+    GRT_CUDA(c, alloc_photons(c, total), "alloc photons");
+    drop_photons(c);  // until the packets are there
     GRT_CUDA(c, c->disk_offsets.alloc(ncell + 1), "alloc offsets");
     GRT_CUDA(c, cudaMemcpy(c->disk_offsets.ptr, off.data(), (ncell + 1) * sizeof(unsigned long long),
                            cudaMemcpyHostToDevice), "H2D offsets");
-    ++c->generation;
-    c->n = total;
-    c->images.clear();
-    c->image_start.clear();
-    c->batched = false;
-    c->have_images = false;
-    c->bproducts_valid = false;
-    c->adj_ready = false;
     grt::DiskInitArgs a{};
     a.ph = c->ph.view();
     a.n = total;
@@ -1373,7 +1399,7 @@ grt_status grt_init_disk_photons(grt_ctx* c, uint64_t id_offset, uint64_t* n_pho
     a.id_offset = id_offset;
     a.dlambda0 = p.initial_step;
     GRT_CUDA(c, grt::launch_init_disk(a, c->stream), "init_disk_photons");
-    c->initial_terminated = 0;
+    c->n = total;
     if (total > 0) {
         grt_status st = count_initial_terminated(c);
         if (st != GRT_OK) return st;

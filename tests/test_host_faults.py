@@ -93,3 +93,39 @@ def test_buffers_shorter_than_the_grid_are_refused(fake, tmp_path, directory):
             ctx.adjoint_image_I(np.zeros((4, 4)), (cells - 1,))
         ctx.adjoint_image_I_device(dL, whole, DeviceArray(fake, cells))
         assert ctx.adjoint_image_I(np.zeros((4, 4)), GRID)[0].shape == GRID
+
+
+@pytest.mark.parametrize("what", ["random", "pixels", "batch", "upload", "disk"])
+def test_a_failed_initialisation_leaves_no_photons(fake, what):
+    """... so that no later call traces the photons, images or queue order of the set before it."""
+    p = image(10)
+    with lib.Context(p) as ctx:
+        ctx.upload_grid(fluid())
+        ctx.init_image_photons(10, 10)
+        ctx.run()
+        assert launches(fake, "trace 1")[-1].split("order=")[1] == "99"
+        if what in ("random", "pixels"):
+            fake.fake_fail_init(1)
+        else:
+            fake.fake_limit(fake.fake_used())
+        with pytest.raises(lib.GrtError):
+            if what == "random":
+                ctx.init_image_photons_random(50)
+            elif what == "pixels":
+                ctx.init_image_photons(5, 5)
+            elif what == "batch":
+                ctx.init_image_batch([abi.ImageSpec.from_params(p, 5, 5)] * 2)
+            elif what == "upload":
+                ctx.upload_photons(abi.PhotonArrays(101))
+            else:
+                ctx.init_disk_photons()
+        fake.fake_reset(1 << 34)
+        assert ctx.n == 0 and ctx.run()["n_terminated"] == 0 and not launches(fake, "trace")
+        with pytest.raises(lib.GrtError):
+            ctx.render_graph()
+        # and the next one starts afresh
+        ctx.init_image_photons_random(50)
+        ctx.run()
+        ctx.init_image_photons(10, 10)
+        ctx.run()
+        assert [line.split("order=")[1] for line in launches(fake, "trace 1")] == ["49", "99"]
