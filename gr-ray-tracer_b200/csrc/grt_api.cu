@@ -1176,11 +1176,16 @@ bool split_legs(const grt_ctx* c) { return c->lc.split_legs != 0 && c->p.mode ==
 // and the instruction cache do.  Trace ms at 2 / 3 / 4 blocks: 1.3e4 packets
 // 2.77 / 2.90 / 3.77, 1.1e5 4.50 / 4.84 / 6.02, 3.4e5 8.70 / 8.50 / 9.75, 5.7e5
 // 13.5 / 12.6 / 14.2, 2.07e6 42.5 / 38.0 / 41.5: 3 above eight packets for
-// every lane of 2 blocks, 2 below.
+// every lane of 2 blocks, 2 below.  That holds while a sample is a few axis reads.
+// On a grid that is not separable its scans of the coordinate arrays are most of a
+// call, and warps hide their latency: as in image mode (64 x 32 x 32, 60 calls,
+// no scattering, run ms at 2 / 3 / 4: 1.5e5 packets 40.0 / 31.1 / 29.9, 3.2e6
+// 674 / 480 / 416).
 int trace_blocks_per_sm(const grt_ctx* c, unsigned long long queue) {
     if (c->lc.blocks_per_sm) return c->lc.blocks_per_sm;
     const unsigned long long lanes = static_cast<unsigned long long>(c->sm_count) * 128;
-    if (c->p.mode == GRT_MODE_DISK) return queue <= 8 * 2 * lanes ? 2 : 3;
+    const bool scans = c->fluid_available && !c->separable;
+    if (c->p.mode == GRT_MODE_DISK && !scans) return queue <= 8 * 2 * lanes ? 2 : 3;
     for (int b = 2; b < 4; ++b)
         if (lanes * b >= queue) return b;
     return 4;

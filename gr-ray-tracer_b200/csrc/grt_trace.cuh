@@ -883,9 +883,13 @@ GRT_DEV void trace_body(const KParams& kp, const Axes& ax, const KStore& kk) {
             // for one lane as for many.  Once a quarter of the live lanes wait
             // (so that a lone lane never does) they scatter together.  One by
             // one, some lane of nearly every warp iteration held the other 31:
-            // 2.07e6 packets 63.1 ms, with a scattering turned off 21.9.
+            // 2.07e6 packets 63.1 ms, with a scattering turned off 21.9.  On a
+            // grid that is not separable the lookup costs more than the tetrad,
+            // and a packet that misses a turn of it pays more than it saves (at
+            // the same launch shapes, waiting / not: 1.5e4 packets 14.8 / 12.5 ms,
+            // 1.5e5 43.8 / 38.5, 3.2e6 628 / 587): none waits there.
             const unsigned waiting = __ballot_sync(kFull, L.idx >= 0 && L.scatter_cell >= 0);
-            if (4 * __popc(waiting) >= __popc(active)) {
+            if (4 * __popc(waiting) >= (kp.grid.separable ? __popc(active) : 1)) {
                 if (L.idx >= 0 && L.scatter_cell >= 0) {
                     scatter_lane<RAW>(kp, L, L.scatter_cell, kp.step0 + L.calls - 1);
                     L.scatter_cell = -1;

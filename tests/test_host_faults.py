@@ -129,3 +129,20 @@ def test_a_failed_initialisation_leaves_no_photons(fake, what):
         ctx.init_image_photons(10, 10)
         ctx.run()
         assert [line.split("order=")[1] for line in launches(fake, "trace 1")] == ["49", "99"]
+
+
+@pytest.mark.parametrize("separable,norm,blocks", [(True, 500.0, 2), (False, 500.0, 4), (False, 2.0, 2)])
+def test_disk_blocks_by_the_grid(fake, separable, norm, blocks):
+    """Two or three blocks a multiprocessor are enough where a sample is a few reads of the axes; the scans of a grid
+    that is not separable want every packet resident that can be."""
+    w = workloads.DiskWorkload("disk", (24, 16, 16), 0.9, norm)
+    grid = torus.benchmark_torus(*w.grid, spin=w.spin)
+    if not separable:
+        grid = dict(grid, **{"theta.npy": grid["theta.npy"] + 1e-4 * np.sin(grid["r.npy"])})
+    with lib.Context(w.params()) as ctx:
+        ctx.upload_grid(grid)
+        n = ctx.init_disk_photons()
+        assert n <= 148 * 2 * 128 if norm < 100 else 148 * 3 * 128 < n <= 8 * 2 * 148 * 128
+        ctx.run()
+    (line,) = launches(fake, "trace 3")
+    assert f"blocks={blocks} " in line
