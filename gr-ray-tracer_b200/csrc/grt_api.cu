@@ -244,6 +244,21 @@ grt_status cuda_fail(grt_ctx* c, cudaError_t e, const char* what) {
         if (e_ != cudaSuccess) return cuda_fail(ctx, e_, what); \
     } while (0)
 
+// Allocates a buffer that a call cannot do without.  When there is no memory
+// for it, what the context holds beside such buffers goes: the adjoint's record
+// (it traces every ray again instead) and the scratch of a screen order.
+template <class Buf>
+cudaError_t room_for(grt_ctx* c, Buf& buf, size_t n) {
+    const cudaError_t e = buf.alloc(n);
+    if (e != cudaErrorMemoryAllocation || !(c->adj_full.ptr || c->screen_scratch.ptr)) return e;
+    cudaGetLastError();
+    c->adj_full.release();
+    c->adj_full_cap = 0;
+    c->adj_stale = true;
+    c->screen_scratch.release();
+    return buf.alloc(n);
+}
+
 // fluid_frame.hpp:28-48 on the host (sines and cosines of the cell's angles by
 // glibc, exactly the reference's arithmetic), then the [units] scale, as sample_scattering_fluid applies it
 // per step (scattering.hpp:223-241).
@@ -581,13 +596,13 @@ grt_status grt_upload_grid(grt_ctx* c, size_t nr, size_t nth, size_t nph, const 
         bv[2 * q] = make_double2(b[0], b[1]);
         bv[2 * q + 1] = make_double2(b[2], b[3]);
     }
-    GRT_CUDA(c, c->rho_t.alloc(ncell), "alloc rho_t");
-    GRT_CUDA(c, c->vel.alloc(2 * ncell), "alloc vel");
-    GRT_CUDA(c, c->mag.alloc(2 * ncell), "alloc mag");
-    GRT_CUDA(c, c->r_axis.alloc(nr), "alloc axis");
-    GRT_CUDA(c, c->th_axis.alloc(nth), "alloc axis");
-    GRT_CUDA(c, c->ph_axis.alloc(nph), "alloc axis");
-    GRT_CUDA(c, c->cell_pos.alloc(3 * ncell), "alloc positions");
+    GRT_CUDA(c, room_for(c, c->rho_t, ncell), "alloc rho_t");
+    GRT_CUDA(c, room_for(c, c->vel, 2 * ncell), "alloc vel");
+    GRT_CUDA(c, room_for(c, c->mag, 2 * ncell), "alloc mag");
+    GRT_CUDA(c, room_for(c, c->r_axis, nr), "alloc axis");
+    GRT_CUDA(c, room_for(c, c->th_axis, nth), "alloc axis");
+    GRT_CUDA(c, room_for(c, c->ph_axis, nph), "alloc axis");
+    GRT_CUDA(c, room_for(c, c->cell_pos, 3 * ncell), "alloc positions");
     GRT_CUDA(c, cudaMemcpy(c->cell_pos.ptr, pos.data(), 3 * ncell * sizeof(double), cudaMemcpyHostToDevice),
              "H2D positions");
     GRT_CUDA(c, cudaMemcpy(c->rho_t.ptr, rt.data(), ncell * sizeof(double2), cudaMemcpyHostToDevice), "H2D grid");
@@ -602,17 +617,17 @@ grt_status grt_upload_grid(grt_ctx* c, size_t nr, size_t nth, size_t nph, const 
         grt::axes::half_spans(ra.data(), nr, 0, rh.data());
         grt::axes::half_spans(ta.data(), nth, 1, th_h.data());
         grt::axes::half_spans(pa.data(), nph, 2, ph_h.data());
-        GRT_CUDA(c, c->r_half.alloc(nr), "alloc half");
-        GRT_CUDA(c, c->th_half.alloc(nth), "alloc half");
-        GRT_CUDA(c, c->ph_half.alloc(nph), "alloc half");
+        GRT_CUDA(c, room_for(c, c->r_half, nr), "alloc half");
+        GRT_CUDA(c, room_for(c, c->th_half, nth), "alloc half");
+        GRT_CUDA(c, room_for(c, c->ph_half, nph), "alloc half");
         GRT_CUDA(c, cudaMemcpy(c->r_half.ptr, rh.data(), nr * sizeof(double), cudaMemcpyHostToDevice), "H2D half");
         GRT_CUDA(c, cudaMemcpy(c->th_half.ptr, th_h.data(), nth * sizeof(double), cudaMemcpyHostToDevice), "H2D half");
         GRT_CUDA(c, cudaMemcpy(c->ph_half.ptr, ph_h.data(), nph * sizeof(double), cudaMemcpyHostToDevice), "H2D half");
     }
     if (!sep) {
-        GRT_CUDA(c, c->r3.alloc(ncell), "alloc r3");
-        GRT_CUDA(c, c->th3.alloc(ncell), "alloc th3");
-        GRT_CUDA(c, c->ph3.alloc(ncell), "alloc ph3");
+        GRT_CUDA(c, room_for(c, c->r3, ncell), "alloc r3");
+        GRT_CUDA(c, room_for(c, c->th3, ncell), "alloc th3");
+        GRT_CUDA(c, room_for(c, c->ph3, ncell), "alloc ph3");
         GRT_CUDA(c, cudaMemcpy(c->r3.ptr, r, ncell * sizeof(double), cudaMemcpyHostToDevice), "H2D r3");
         GRT_CUDA(c, cudaMemcpy(c->th3.ptr, th, ncell * sizeof(double), cudaMemcpyHostToDevice), "H2D th3");
         GRT_CUDA(c, cudaMemcpy(c->ph3.ptr, ph, ncell * sizeof(double), cudaMemcpyHostToDevice), "H2D ph3");
@@ -699,7 +714,7 @@ static void drop_photons(grt_ctx* c) {
 
 // Room for n photons, or none at all.
 static cudaError_t alloc_photons(grt_ctx* c, size_t n) {
-    const cudaError_t e = c->ph.alloc(n);
+    const cudaError_t e = room_for(c, c->ph, n);
     if (e != cudaSuccess) drop_photons(c);
     return e;
 }
@@ -907,7 +922,7 @@ grt_status set_tile_orders(grt_ctx* c, const std::vector<unsigned long long>& st
     ord.reserve(c->n);
     for (size_t k = 0; k + 1 < start.size(); ++k)
         append_tile_order(ord, start[k], c->images[k].nx, (start[k + 1] - start[k]) / c->images[k].nx);
-    GRT_CUDA(c, c->order_ph.alloc(ord.size()), "alloc queue order");
+    GRT_CUDA(c, room_for(c, c->order_ph, ord.size()), "alloc queue order");
     GRT_CUDA(c, cudaMemcpy(c->order_ph.ptr, ord.data(), ord.size() * sizeof(unsigned), cudaMemcpyHostToDevice),
              "H2D queue order");
     c->order_ph_ok = ord.size() == c->n;
@@ -917,7 +932,7 @@ grt_status set_tile_orders(grt_ctx* c, const std::vector<unsigned long long>& st
             const grt_image_spec& lead = c->images[chan[gchan[g]]];
             append_tile_order(ord, qstart[g], lead.nx, lead.ny);
         }
-        GRT_CUDA(c, c->order_geo.alloc(ord.size()), "alloc queue order");
+        GRT_CUDA(c, room_for(c, c->order_geo, ord.size()), "alloc queue order");
         GRT_CUDA(c, cudaMemcpy(c->order_geo.ptr, ord.data(), ord.size() * sizeof(unsigned), cudaMemcpyHostToDevice),
                  "H2D queue order");
         c->order_geo_ok = ord.size() == c->geodesics;
@@ -959,7 +974,7 @@ grt_status lay_out_images(grt_ctx* c, const grt_image_spec* specs, size_t nimage
                           const std::vector<unsigned long long>& start, uint64_t id_offset, bool batched,
                           double forward_back, uint64_t row0, uint64_t nrows, bool random_screen) {
     const unsigned long long total = start[nimages];
-    GRT_CUDA(c, c->ph.alloc(total), "alloc photons");
+    GRT_CUDA(c, room_for(c, c->ph, total), "alloc photons");
     ++c->generation;
     c->n = total;
     c->initial_terminated = 0;
@@ -984,8 +999,8 @@ grt_status lay_out_images(grt_ctx* c, const grt_image_spec* specs, size_t nimage
                                       sp.emission_coefficient);
         }
         (void)p;
-        GRT_CUDA(c, c->images_dev.alloc(nimages), "alloc image table");
-        GRT_CUDA(c, c->image_start_dev.alloc(nimages + 1), "alloc image table");
+        GRT_CUDA(c, room_for(c, c->images_dev, nimages), "alloc image table");
+        GRT_CUDA(c, room_for(c, c->image_start_dev, nimages + 1), "alloc image table");
         GRT_CUDA(c, cudaMemcpy(c->images_dev.ptr, tab.data(), nimages * sizeof(grt::KImage), cudaMemcpyHostToDevice),
                  "H2D image table");
         GRT_CUDA(c, cudaMemcpy(c->image_start_dev.ptr, start.data(), (nimages + 1) * sizeof(unsigned long long),
@@ -1018,10 +1033,10 @@ grt_status lay_out_images(grt_ctx* c, const grt_image_spec* specs, size_t nimage
         }
         c->ngroups = static_cast<int>(groups.size());
         c->geodesics = qstart.back();
-        if (c->groups_share) GRT_CUDA(c, c->share_state.alloc(c->geodesics), "alloc share state");
-        GRT_CUDA(c, c->group_qstart_dev.alloc(qstart.size()), "alloc groups");
-        GRT_CUDA(c, c->group_chan_dev.alloc(gchan.size()), "alloc groups");
-        GRT_CUDA(c, c->chan_img_dev.alloc(chan.size()), "alloc groups");
+        if (c->groups_share) GRT_CUDA(c, room_for(c, c->share_state, c->geodesics), "alloc share state");
+        GRT_CUDA(c, room_for(c, c->group_qstart_dev, qstart.size()), "alloc groups");
+        GRT_CUDA(c, room_for(c, c->group_chan_dev, gchan.size()), "alloc groups");
+        GRT_CUDA(c, room_for(c, c->chan_img_dev, chan.size()), "alloc groups");
         GRT_CUDA(c, cudaMemcpy(c->group_qstart_dev.ptr, qstart.data(), qstart.size() * sizeof(unsigned long long),
                                cudaMemcpyHostToDevice), "H2D groups");
         GRT_CUDA(c, cudaMemcpy(c->group_chan_dev.ptr, gchan.data(), gchan.size() * sizeof(int), cudaMemcpyHostToDevice),
@@ -1115,9 +1130,9 @@ grt_status launch_all_products(grt_ctx* c) {
     const size_t nimg = c->images.size(), bins = c->p.spectrum_bins;
     c->bimage_off.assign(nimg + 1, 0);
     for (size_t k = 0; k < nimg; ++k) c->bimage_off[k + 1] = c->bimage_off[k] + 4 * c->images[k].nx * c->images[k].ny;
-    GRT_CUDA(c, c->bimage.alloc(c->bimage_off[nimg]), "alloc products");
-    GRT_CUDA(c, c->bspectrum.alloc(nimg * bins), "alloc products");
-    GRT_CUDA(c, c->barrived.alloc(nimg), "alloc products");
+    GRT_CUDA(c, room_for(c, c->bimage, c->bimage_off[nimg]), "alloc products");
+    GRT_CUDA(c, room_for(c, c->bspectrum, nimg * bins), "alloc products");
+    GRT_CUDA(c, room_for(c, c->barrived, nimg), "alloc products");
     if (nimg == 0) return GRT_OK;
     GRT_CUDA(c, cudaMemsetAsync(c->bimage.ptr, 0, c->bimage_off[nimg] * sizeof(double), c->stream), "memset");
     if (bins) GRT_CUDA(c, cudaMemsetAsync(c->bspectrum.ptr, 0, nimg * bins * sizeof(double), c->stream), "memset");
@@ -1207,7 +1222,7 @@ bool hands_on(const grt_ctx* c, unsigned long long queue) {
 // launch or graph capture.
 grt_status prepare_trace_buffers(grt_ctx* c, unsigned long long queue) {
     if (split_legs(c)) {
-        GRT_CUDA(c, c->calls_carry.alloc(queue), "alloc call carry");
+        GRT_CUDA(c, room_for(c, c->calls_carry, queue), "alloc call carry");
         if (hands_on(c, queue) && c->stragglers.alloc(queue) != cudaSuccess) cudaGetLastError();  // done without
     }
     return GRT_OK;
@@ -1314,7 +1329,7 @@ grt_status grt_init_image_photons(grt_ctx* c, uint64_t nx, uint64_t ny, uint64_t
     if (!c) return GRT_EINVAL;
     const grt_image_spec sp = spec_from_params(c->p, nx, ny);
     if (nx * ny == 0) {
-        GRT_CUDA(c, c->ph.alloc(0), "alloc photons");
+        GRT_CUDA(c, room_for(c, c->ph, 0), "alloc photons");
         c->n = 0;
         c->images.clear();
         c->image_start.clear();
@@ -1376,7 +1391,7 @@ grt_status grt_init_disk_photons(grt_ctx* c, uint64_t id_offset, uint64_t* n_pho
     if (total > (1ull << 36)) return fail(c, GRT_EINVAL, "disk packet count too large: " + std::to_string(total));
     GRT_CUDA(c, alloc_photons(c, total), "alloc photons");
     drop_photons(c);  // until the packets are there
-    GRT_CUDA(c, c->disk_offsets.alloc(ncell + 1), "alloc offsets");
+    GRT_CUDA(c, room_for(c, c->disk_offsets, ncell + 1), "alloc offsets");
     GRT_CUDA(c, cudaMemcpy(c->disk_offsets.ptr, off.data(), (ncell + 1) * sizeof(unsigned long long),
                            cudaMemcpyHostToDevice), "H2D offsets");
     grt::DiskInitArgs a{};
@@ -1678,9 +1693,9 @@ grt_status grt_render_graph(grt_ctx* c, grt_run_stats* stats) {
         const size_t nimg = c->images.size(), bins = p.spectrum_bins;
         size_t pix = 0;
         for (const auto& sp : c->images) pix += 4 * sp.nx * sp.ny;
-        GRT_CUDA(c, c->bimage.alloc(pix), "alloc products");
-        GRT_CUDA(c, c->bspectrum.alloc(nimg * bins), "alloc products");
-        GRT_CUDA(c, c->barrived.alloc(nimg), "alloc products");
+        GRT_CUDA(c, room_for(c, c->bimage, pix), "alloc products");
+        GRT_CUDA(c, room_for(c, c->bspectrum, nimg * bins), "alloc products");
+        GRT_CUDA(c, room_for(c, c->barrived, nimg), "alloc products");
         grt::KParams kp = make_kparams(c);
         {
             const grt_status bs = prepare_trace_buffers(c, kp.n);
@@ -1819,9 +1834,9 @@ grt_status grt_render_async(grt_ctx* c, const grt_photon_soa* s, grt_image_produ
         if (bs != GRT_OK) return bs;
         size_t pix = 0;
         for (const auto& sp : c->images) pix += 4 * sp.nx * sp.ny;
-        GRT_CUDA(c, c->bimage.alloc(pix), "alloc products");
-        GRT_CUDA(c, c->bspectrum.alloc(nimages * p.spectrum_bins), "alloc products");
-        GRT_CUDA(c, c->barrived.alloc(nimages), "alloc products");
+        GRT_CUDA(c, room_for(c, c->bimage, pix), "alloc products");
+        GRT_CUDA(c, room_for(c, c->bspectrum, nimages * p.spectrum_bins), "alloc products");
+        GRT_CUDA(c, room_for(c, c->barrived, nimages), "alloc products");
     }
     c->bproducts_valid = false;
     c->adj_ready = false;
@@ -1876,13 +1891,13 @@ grt_status grt_set_cell_multipliers(grt_ctx* c, const double* m_abs, const doubl
     c->adj_ready = false;
     c->has_m_abs = c->has_m_emis = false;
     if (m_abs) {
-        GRT_CUDA(c, c->m_abs.alloc(ncell), "alloc multipliers");
+        GRT_CUDA(c, room_for(c, c->m_abs, ncell), "alloc multipliers");
         GRT_CUDA(c, cudaMemcpyAsync(c->m_abs.ptr, m_abs, ncell * sizeof(double), cudaMemcpyDefault, c->stream),
                  "copy multipliers");
         c->has_m_abs = true;
     }
     if (m_emis) {
-        GRT_CUDA(c, c->m_emis.alloc(ncell), "alloc multipliers");
+        GRT_CUDA(c, room_for(c, c->m_emis, ncell), "alloc multipliers");
         GRT_CUDA(c, cudaMemcpyAsync(c->m_emis.ptr, m_emis, ncell * sizeof(double), cudaMemcpyDefault, c->stream),
                  "copy multipliers");
         c->has_m_emis = true;
@@ -1933,20 +1948,25 @@ grt_status grt_forward_checkpointed(grt_ctx* c, int64_t K, grt_run_stats* stats)
     const int threads = 128;
     const long long want_blocks = (static_cast<long long>(n) + threads - 1) / threads;
     const int blocks = static_cast<int>(std::max(1ll, std::min<long long>(want_blocks, 8ll * c->sm_count)));
-    GRT_CUDA(c, c->ckpt.alloc(n * cap * 16), "alloc checkpoints");
-    GRT_CUDA(c, c->nckpt.alloc(std::max<size_t>(n, 1)), "alloc checkpoints");
-    GRT_CUDA(c, c->call0.alloc(std::max<size_t>(n, 1)), "alloc checkpoints");
-    GRT_CUDA(c, c->adj_overflow.alloc(2), "alloc checkpoints");  // overflow, rays not recorded
-    GRT_CUDA(c, c->adj_nfull.alloc(std::max<size_t>(n, 1)), "alloc checkpoints");
+    GRT_CUDA(c, room_for(c, c->ckpt, n * cap * 16), "alloc checkpoints");
+    GRT_CUDA(c, room_for(c, c->nckpt, std::max<size_t>(n, 1)), "alloc checkpoints");
+    GRT_CUDA(c, room_for(c, c->call0, std::max<size_t>(n, 1)), "alloc checkpoints");
+    GRT_CUDA(c, room_for(c, c->adj_overflow, 2), "alloc checkpoints");  // overflow, rays not recorded
+    GRT_CUDA(c, room_for(c, c->adj_nfull, std::max<size_t>(n, 1)), "alloc checkpoints");
+    GRT_CUDA(c, room_for(c, c->tape, static_cast<size_t>(blocks) * threads * K * 6), "alloc tape");
     // the record of every ray's transfer updates, as far as the memory set
-    // aside for it goes; rays with more updates are traced again by the adjoint
+    // aside for it goes; rays with more updates are traced again by the adjoint.
+    // Last, and at most half of what is then free: the pass can do without it.
     c->adj_full_cap = static_cast<int>(std::min<unsigned long long>(
         std::min<int64_t>(p.max_steps, kRecordedSteps), kRecordBytes / (48ull * std::max<size_t>(n, 1))));
-    if (c->adj_full.alloc(n * c->adj_full_cap * 6) != cudaSuccess) {
+    const size_t record = n * c->adj_full_cap * 6;
+    size_t free_bytes = 0, total_bytes = 0;
+    if (record > c->adj_full.count &&
+        ((c->adj_full.release(), cudaMemGetInfo(&free_bytes, &total_bytes)) != cudaSuccess ||
+         record * sizeof(double) > free_bytes / 2 || c->adj_full.alloc(record) != cudaSuccess)) {
         cudaGetLastError();
         c->adj_full_cap = 0;
     }
-    GRT_CUDA(c, c->tape.alloc(static_cast<size_t>(blocks) * threads * K * 6), "alloc tape");
     c->adj_K = static_cast<int>(K);
     c->adj_cap = static_cast<int>(cap);
     if (n == 0) {
@@ -1995,9 +2015,9 @@ grt_status grt_adjoint_image_I(grt_ctx* c, const double* dL_dI, double* g_abs, d
     const grt_params& p = c->p;
     const size_t ncell = static_cast<size_t>(c->nr) * c->nth * c->nph;
     const size_t npix = p.image_nx * p.image_ny;
-    GRT_CUDA(c, c->dLdI.alloc(std::max<size_t>(npix, 1)), "alloc");
-    GRT_CUDA(c, c->g_abs.alloc(std::max<size_t>(ncell, 1)), "alloc");
-    GRT_CUDA(c, c->g_emis.alloc(std::max<size_t>(ncell, 1)), "alloc");
+    GRT_CUDA(c, room_for(c, c->dLdI, std::max<size_t>(npix, 1)), "alloc");
+    GRT_CUDA(c, room_for(c, c->g_abs, std::max<size_t>(ncell, 1)), "alloc");
+    GRT_CUDA(c, room_for(c, c->g_emis, std::max<size_t>(ncell, 1)), "alloc");
     GRT_CUDA(c, cudaMemcpyAsync(c->dLdI.ptr, dL_dI, npix * sizeof(double), cudaMemcpyDefault, c->stream), "copy dL/dI");
     GRT_CUDA(c, cudaMemsetAsync(c->g_abs.ptr, 0, std::max<size_t>(ncell, 1) * sizeof(double), c->stream), "memset");
     GRT_CUDA(c, cudaMemsetAsync(c->g_emis.ptr, 0, std::max<size_t>(ncell, 1) * sizeof(double), c->stream), "memset");
@@ -2096,7 +2116,7 @@ grt_status grt_get_image_products(grt_ctx* c, grt_image_products* out) {
     const grt_params& p = c->p;
     const size_t npix = p.image_nx * p.image_ny, bins = p.spectrum_bins;
     if (!products_complete(out)) return fail(c, GRT_EINVAL, "null image product buffer");
-    GRT_CUDA(c, c->image.alloc(4 * npix + bins + 1), "alloc image");
+    GRT_CUDA(c, room_for(c, c->image, 4 * npix + bins + 1), "alloc image");
     grt_status st = launch_products(c, 0, c->n, p.image_nx, p.image_ny, p.camera_width, p.camera_height, c->image.ptr);
     if (st != GRT_OK) return st;
     return copy_products_out(c, npix, bins, out);
@@ -2170,7 +2190,7 @@ grt_status write_output_step(grt_ctx* c, const OutputPlan& plan, int64_t step) {
     g.count = count;
     g.stride = plan.stride;
     if (bytes > 0) {
-        GRT_CUDA(c, c->out_stage.alloc(bytes), "alloc output stage");
+        GRT_CUDA(c, room_for(c, c->out_stage, bytes), "alloc output stage");
         if (c->host_out_bytes < bytes) {
             if (c->host_out) cudaFreeHost(c->host_out);
             c->host_out = nullptr;

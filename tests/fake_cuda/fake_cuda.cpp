@@ -90,6 +90,11 @@ cudaError_t cudaFree(void* p) {
     std::free(p);
     return cudaSuccess;
 }
+cudaError_t cudaMemGetInfo(size_t* free_bytes, size_t* total) {
+    *total = limit;
+    *free_bytes = limit > used ? limit - used : 0;
+    return cudaSuccess;
+}
 cudaError_t cudaMallocHost(void** p, size_t n) {
     if (refuse_pinned) return cudaErrorMemoryAllocation;
     char* q = static_cast<char*>(std::malloc(n ? n : 1));

@@ -146,3 +146,48 @@ def test_disk_blocks_by_the_grid(fake, separable, norm, blocks):
         ctx.run()
     (line,) = launches(fake, "trace 3")
     assert f"blocks={blocks} " in line
+
+
+def differentiate(fake, ctx, px, squeeze=False):
+    """The calls of one differentiable render; with squeeze, no memory is left once the forward pass has returned."""
+    ctx.set_cell_multipliers(np.ones(GRID), np.ones(GRID))
+    ctx.init_image_forward_photons(px, px, 60.0)
+    ctx.forward_checkpointed(64)
+    held = fake.fake_used()
+    if squeeze:
+        fake.fake_limit(held)
+    ctx.image_products()
+    ctx.adjoint_image_I(np.ones((px, px)), GRID)
+    return held
+
+
+def test_the_record_of_updates_leaves_memory_to_what_is_needed(fake):
+    px = 40
+    record = px * px * 128 * 48
+    with lib.Context(image(px)) as ctx:
+        ctx.upload_grid(fluid())
+        differentiate(fake, ctx, px)
+        assert launches(fake, "forward") == ["forward cap=128"] and launches(fake, "sweep") == ["sweep"]
+        needed = fake.fake_used() - record
+    # room for all but the record: rays are traced again
+    for memory in (needed, needed + record // 2):
+        fake.fake_reset(memory)
+        with lib.Context(image(px)) as ctx:
+            ctx.upload_grid(fluid())
+            differentiate(fake, ctx, px)
+            assert launches(fake, "forward") == ["forward cap=0"]
+    # a record that is there goes when another buffer needs the room, in the
+    # same render and in a larger one after it
+    fake.fake_reset(1 << 34)
+    with lib.Context(image(px)) as ctx:
+        ctx.upload_grid(fluid())
+        held = differentiate(fake, ctx, px, squeeze=True)
+        assert launches(fake, "forward") == ["forward cap=128"]
+        assert launches(fake, "reverse") and not launches(fake, "sweep")
+        assert fake.fake_used() <= held - record // 2
+        fake.fake_reset(1 << 34)
+        differentiate(fake, ctx, px)
+        fake.fake_limit(fake.fake_used())
+        ctx.init_image_photons(2 * px, px)  # 146 bytes a photon where the record held 6144
+        ctx.init_image_photons_random(px * px)
+        ctx.run()
