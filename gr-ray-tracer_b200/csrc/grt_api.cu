@@ -2070,10 +2070,6 @@ grt_status grt_adjoint_image_I(grt_ctx* c, const double* dL_dI, double* g_abs, d
 // x 256 image's 260, and added 2 to 7 ms to a context's first frame at any size.
 constexpr size_t kStageMax = 640u << 10;
 static grt_status copy_products_out(grt_ctx* c, size_t npix, size_t bins, grt_image_products* out) {
-    cudaPointerAttributes at;
-    const bool pageable = cudaPointerGetAttributes(&at, out->image_I) != cudaSuccess ||
-                          at.type == cudaMemoryTypeUnregistered;
-    cudaGetLastError();
     struct Part {
         void* dst;
         size_t bytes;
@@ -2084,7 +2080,19 @@ static grt_status copy_products_out(grt_ctx* c, size_t npix, size_t bins, grt_im
     const unsigned char* src = reinterpret_cast<const unsigned char*>(c->image.ptr);
     const size_t total = (4 * npix + bins + 1) * sizeof(double);
     fill_spectrum_frequencies(c->p, out->spectrum_frequency_hz);
-    if (!pageable || total > kStageMax) {
+    cudaPointerAttributes at;
+    const bool pageable = cudaPointerGetAttributes(&at, out->image_I) != cudaSuccess ||
+                          at.type == cudaMemoryTypeUnregistered;
+    bool staged = pageable && total <= kStageMax;
+    if (staged && c->host_stage_bytes < total) {
+        if (c->host_stage) cudaFreeHost(c->host_stage);
+        c->host_stage = nullptr;
+        c->host_stage_bytes = 0;
+        staged = cudaMallocHost(reinterpret_cast<void**>(&c->host_stage), total) == cudaSuccess;
+        if (staged) c->host_stage_bytes = total;
+    }
+    cudaGetLastError();
+    if (!staged) {  // page-locked arrays, large blocks, or no memory to pin
         for (const Part& part : parts) {
             if (part.bytes)
                 GRT_CUDA(c, cudaMemcpyAsync(part.dst, src, part.bytes, cudaMemcpyDeviceToHost, c->stream), "D2H products");
@@ -2092,13 +2100,6 @@ static grt_status copy_products_out(grt_ctx* c, size_t npix, size_t bins, grt_im
         }
         GRT_CUDA(c, cudaStreamSynchronize(c->stream), "products");
         return GRT_OK;
-    }
-    if (c->host_stage_bytes < total) {
-        if (c->host_stage) cudaFreeHost(c->host_stage);
-        c->host_stage = nullptr;
-        c->host_stage_bytes = 0;
-        GRT_CUDA(c, cudaMallocHost(reinterpret_cast<void**>(&c->host_stage), total), "alloc products stage");
-        c->host_stage_bytes = total;
     }
     GRT_CUDA(c, cudaMemcpyAsync(c->host_stage, src, total, cudaMemcpyDeviceToHost, c->stream), "D2H products");
     GRT_CUDA(c, cudaStreamSynchronize(c->stream), "products");

@@ -191,3 +191,14 @@ def test_the_record_of_updates_leaves_memory_to_what_is_needed(fake):
         ctx.init_image_photons(2 * px, px)  # 146 bytes a photon where the record held 6144
         ctx.init_image_photons_random(px * px)
         ctx.run()
+
+
+def test_products_without_memory_to_pin_are_copied_directly(fake):
+    with lib.Context(image(16)) as ctx:
+        ctx.upload_grid(fluid())
+        ctx.init_image_photons(16, 16)
+        ctx.run()
+        fake.fake_refuse_pinned(1)
+        ctx.image_products()
+        fake.fake_refuse_pinned(0)
+        ctx.image_products()
