@@ -2080,10 +2080,11 @@ static grt_status copy_products_out(grt_ctx* c, size_t npix, size_t bins, grt_im
     const unsigned char* src = reinterpret_cast<const unsigned char*>(c->image.ptr);
     const size_t total = (4 * npix + bins + 1) * sizeof(double);
     fill_spectrum_frequencies(c->p, out->spectrum_frequency_hz);
-    cudaPointerAttributes at;
-    const bool pageable = cudaPointerGetAttributes(&at, out->image_I) != cudaSuccess ||
-                          at.type == cudaMemoryTypeUnregistered;
-    bool staged = pageable && total <= kStageMax;
+    bool staged = total <= kStageMax;
+    for (const Part& part : parts) {
+        cudaPointerAttributes at;
+        staged = staged && (cudaPointerGetAttributes(&at, part.dst) != cudaSuccess || at.type == cudaMemoryTypeUnregistered);
+    }
     if (staged && c->host_stage_bytes < total) {
         if (c->host_stage) cudaFreeHost(c->host_stage);
         c->host_stage = nullptr;
@@ -2092,7 +2093,7 @@ static grt_status copy_products_out(grt_ctx* c, size_t npix, size_t bins, grt_im
         if (staged) c->host_stage_bytes = total;
     }
     cudaGetLastError();
-    if (!staged) {  // page-locked arrays, large blocks, or no memory to pin
+    if (!staged) {  // arrays the host may not write, page-locked ones, large blocks, or no memory to pin
         for (const Part& part : parts) {
             if (part.bytes)
                 GRT_CUDA(c, cudaMemcpyAsync(part.dst, src, part.bytes, cudaMemcpyDeviceToHost, c->stream), "D2H products");

@@ -202,3 +202,19 @@ def test_products_without_memory_to_pin_are_copied_directly(fake):
         ctx.image_products()
         fake.fake_refuse_pinned(0)
         ctx.image_products()
+
+
+@pytest.mark.parametrize("field", ["image_I", "image_Q", "spectrum_I", "arrived_count"])
+def test_device_memory_as_a_product_array_is_an_error(fake, field):
+    """... and not written by the host, whichever array it is."""
+    with lib.Context(image(16)) as ctx:
+        ctx.upload_grid(fluid())
+        ctx.init_image_photons(16, 16)
+        ctx.run()
+        arrays = abi.ProductArrays.for_params(ctx.params)
+        out = arrays.struct()
+        ptr = DeviceArray(fake, 16, 16).data_ptr()
+        C.memset(ptr, 7, 16 * 16 * 8)
+        setattr(out, field, C.cast(ptr, type(getattr(out, field))))
+        assert fake.grt_get_image_products(ctx.handle, C.byref(out)) == abi.GRT_ECUDA
+        assert C.string_at(ptr, 16 * 16 * 8) == b"\7" * (16 * 16 * 8)
