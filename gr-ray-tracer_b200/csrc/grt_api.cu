@@ -158,6 +158,7 @@ struct grt_ctx {
     unsigned long long* host_u64 = nullptr;  // pinned
     grt_launch_config lc{128, 0, 8, 32, 1, 0, 0};
     bool lc_set = false;  // the caller chose a launch shape (grt_set_launch_config)
+    bool refill_set = false;  // and in it a refill threshold that is not the mode's own
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // images of the last grt_init_image_photons (one, cameras from p) or
     // grt_init_image_batch call; image k owns photon slots
@@ -292,6 +293,11 @@ constexpr int64_t kWholeRayCalls = 4;
 // stage slots take 42 KB of the 227 KB a block can have).
 constexpr size_t kMaxStagedAxisBytes = 160 * 1024;
 
+// The refill threshold in force.
+int refill_threshold(const grt_ctx* c) {
+    return c->refill_set ? c->lc.refill_threshold : grt::default_refill(c->p.mode == GRT_MODE_IMAGE);
+}
+
 grt::KParams make_kparams(const grt_ctx* c) {
     const grt_params& p = c->p;
     grt::KParams k;
@@ -376,7 +382,7 @@ grt::KParams make_kparams(const grt_ctx* c) {
                                 : (c->order_ph_ok ? c->order_ph.ptr : nullptr);
     k.calls_carry = c->calls_carry.ptr;
     k.counters = c->counters.ptr;
-    k.refill_threshold = c->lc_set ? c->lc.refill_threshold : grt::default_refill(k.image_mode);
+    k.refill_threshold = refill_threshold(c);
     k.grab = c->lc.photons_per_grab;
     k.fp64_radius_sq = 16.0 * p.mass * p.mass + p.spin * p.spin;
     k.fp64_axis_sin2 = 0.01;
@@ -510,6 +516,7 @@ grt_status grt_synchronize(grt_ctx* c) {
 grt_status grt_get_launch_config(const grt_ctx* c, grt_launch_config* cfg) {
     if (!c || !cfg) return GRT_EINVAL;
     *cfg = c->lc;
+    cfg->refill_threshold = refill_threshold(c);
     return GRT_OK;
 }
 
@@ -530,6 +537,8 @@ grt_status grt_set_launch_config(grt_ctx* c, const grt_launch_config* cfg) {
     c->lc = *cfg;
     c->lc.pad = 0;
     c->lc_set = true;
+    // the mode's own threshold, as grt_get_launch_config hands it out, goes on following the mode
+    c->refill_set = cfg->refill_threshold != grt::default_refill(c->p.mode == GRT_MODE_IMAGE);
     ++c->generation;
     return GRT_OK;
 }
@@ -1212,10 +1221,9 @@ int trace_blocks_per_sm(const grt_ctx* c, unsigned long long queue) {
 // 2.1 tiles for every warp 1.92 / 2.00, 3.5 2.83 / 2.86, 5.4 3.82 / 3.75, 8.4
 // 6.01 / 5.84, 13 8.77 / 8.47.
 bool hands_on(const grt_ctx* c, unsigned long long queue) {
-    const int refill = c->lc_set ? c->lc.refill_threshold : grt::default_refill(1);
     const unsigned long long grab = static_cast<unsigned long long>(c->lc.photons_per_grab);
     const unsigned long long warps = 4ull * c->sm_count * trace_blocks_per_sm(c, queue);
-    return refill == 32 && queue < (1ull << 32) && (queue + grab - 1) / grab >= 5 * warps;
+    return refill_threshold(c) == 32 && queue < (1ull << 32) && (queue + grab - 1) / grab >= 5 * warps;
 }
 
 // Device buffers a trace needs besides the photons; allocated before any

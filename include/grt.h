@@ -157,10 +157,12 @@ typedef struct grt_image_products {
     uint64_t* arrived_count;      /* [1] */
 } grt_image_products;
 
-/* Launch shape of the trace kernel: the library's default is {128, 0, 8, 32, 1, 0, 0};
- * grt/autotune.py times the candidates on a workload and picks one.  Until a shape is
- * set (grt_set_launch_config) the refill threshold goes by the mode: 32 (whole tiles)
- * in image mode, 4 in disk mode.  The shape never changes results. */
+/* Launch shape of the trace kernel: the library's default is {128, 0, R, 32, 1, 0, 0} with
+ * a refill threshold R that goes by the mode, 32 (whole tiles) in image mode and 4 in
+ * disk mode.  grt_get_launch_config returns what is in force; a shape that is set
+ * with the mode's own threshold goes on following the mode.  grt/autotune.py times the
+ * candidates on a workload and picks one.  The shape never changes
+ * results. */
 typedef struct grt_launch_config {
     int32_t threads_per_block;    /* 128 (the trace kernels' block size) */
     int32_t blocks_per_sm;        /* 2, 3 or 4 resident blocks per SM: register caps 255 / 170 / 128;
@@ -173,7 +175,9 @@ typedef struct grt_launch_config {
                                      first claims are spread evenly over the SMs. */
     int32_t split_legs;           /* image mode: 1 = the backward legs, the packet generation at first
                                      fluid contact and the rest as three launches (same results, smaller
-                                     loop bodies); 0 = one launch for whole rays */
+                                     loop bodies); 0 = one launch for whole rays.  Until a shape is
+                                     set, chunks of up to 4 calls (termination_percent < 1) take one
+                                     launch; in a shape that is set this holds for every chunk */
     int32_t pad;
     int64_t max_iterations;       /* per-warp loop iterations a trace launch may take before it stops,
                                      writes every photon back at its last call boundary and the run

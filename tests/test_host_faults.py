@@ -218,3 +218,33 @@ def test_device_memory_as_a_product_array_is_an_error(fake, field):
         setattr(out, field, C.cast(ptr, type(getattr(out, field))))
         assert fake.grt_get_image_products(ctx.handle, C.byref(out)) == abi.GRT_ECUDA
         assert C.string_at(ptr, 16 * 16 * 8) == b"\7" * (16 * 16 * 8)
+
+
+def thresholds(fake):
+    return [int(line.split("refill=")[1].split()[0]) for line in launches(fake, "trace")]
+
+
+def test_a_field_of_the_launch_shape_leaves_the_refill_threshold_to_the_mode(fake):
+    disk = workloads.DiskWorkload("disk", GRID, 0.9, 500.0).params()
+    with lib.Context(image(700)) as ctx:
+        ctx.upload_grid(fluid())
+        assert ctx.launch_config()["refill_threshold"] == 32
+        ctx.set_launch_config(max_iterations=10**9)  # gets, changes one field, sets
+        ctx.init_image_photons(700, 700)
+        ctx.run()
+        assert set(thresholds(fake)) == {32}
+        assert [line.split()[1] for line in launches(fake, "trace") if "hands_on" in line] == ["1", "2"]
+        fake.fake_clear()
+        ctx.set_params(disk)
+        assert ctx.launch_config()["refill_threshold"] == 4
+        ctx.init_disk_photons()
+        ctx.run()
+        assert thresholds(fake) == [4]
+        fake.fake_clear()
+        ctx.set_launch_config(refill_threshold=8)  # a threshold of the caller's own stays
+        ctx.run()
+        ctx.set_params(image(700))
+        ctx.init_image_photons(700, 700)
+        ctx.run()
+        assert set(thresholds(fake)) == {8} and not any("hands_on" in line for line in launches(fake, "trace"))
+        assert ctx.launch_config()["refill_threshold"] == 8
