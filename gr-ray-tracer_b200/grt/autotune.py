@@ -46,7 +46,9 @@ def tune(ctx, prepare, key, reps: int = 2, log=None):
     table = []
     best = None
     from .abi import MODE_IMAGE
-    for cfg in candidates(ctx.params.mode == MODE_IMAGE):
+    # the shape in force first: no candidate is taken that is slower than what
+    # the library does by itself
+    for cfg in itertools.chain((ctx.launch_config(),), candidates(ctx.params.mode == MODE_IMAGE)):
         ctx.set_launch_config(**cfg)
         prepare(ctx)
         ctx.run()

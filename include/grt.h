@@ -161,7 +161,7 @@ typedef struct grt_image_products {
  * a refill threshold R that goes by the mode, 32 (whole tiles) in image mode and 4 in
  * disk mode.  grt_get_launch_config returns what is in force; a shape that is set
  * with the mode's own threshold goes on following the mode.  grt/autotune.py times the
- * candidates on a workload and picks one.  The shape never changes
+ * default and its candidates on a workload and picks one.  The shape never changes
  * results. */
 typedef struct grt_launch_config {
     int32_t threads_per_block;    /* 128 (the trace kernels' block size) */

@@ -9,7 +9,7 @@ from pathlib import Path
 import numpy as np
 import pytest
 
-from grt import abi, lib, torus, workloads
+from grt import abi, autotune, lib, torus, workloads
 
 HERE = Path(__file__).resolve().parent
 SRC = HERE.parent / "gr-ray-tracer_b200" / "csrc"
@@ -248,3 +248,26 @@ def test_a_field_of_the_launch_shape_leaves_the_refill_threshold_to_the_mode(fak
         ctx.run()
         assert set(thresholds(fake)) == {8} and not any("hands_on" in line for line in launches(fake, "trace"))
         assert ctx.launch_config()["refill_threshold"] == 8
+
+
+def test_the_tuner_keeps_the_shape_in_force_when_nothing_is_faster(monkeypatch):
+    monkeypatch.setattr(autotune, "_CACHE", {})
+    own = dict(threads_per_block=128, blocks_per_sm=0, refill_threshold=4, photons_per_grab=32, split_legs=1,
+               max_iterations=0)
+
+    class Tuned:
+        params = workloads.DiskWorkload("disk", GRID, 0.9, 2.0).params()
+        shape = dict(own)
+
+        def launch_config(self):
+            return dict(self.shape)
+
+        def set_launch_config(self, **kw):
+            self.shape.update(kw)
+
+        def run(self):
+            return dict(trace_ms=1.0 if self.shape["blocks_per_sm"] == 0 else 2.0)
+
+    ctx = Tuned()
+    best, ms, table = autotune.tune(ctx, lambda c: None, "disk")
+    assert best == own == ctx.shape and ms == 1.0 and len(table) == 1 + len(list(autotune.candidates(False)))
