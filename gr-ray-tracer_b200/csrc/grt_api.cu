@@ -357,6 +357,7 @@ grt::KParams make_kparams(const grt_ctx* c) {
     std::memcpy(g.per, c->lookup.per, sizeof(g.per));
     std::memcpy(g.margin, c->lookup.margin, sizeof(g.margin));
     g.even = c->lookup.even;
+    g.r_fp32 = grt::fp32_lookup_radius(p.spin);
     g.r_certain = p.spin == c->lookup_spin && p.mass == c->lookup_mass ? c->lookup.r_certain : INFINITY;
     k.m_abs = c->has_m_abs ? c->m_abs.ptr : nullptr;
     k.m_emis = c->has_m_emis ? c->m_emis.ptr : nullptr;

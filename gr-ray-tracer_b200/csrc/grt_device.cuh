@@ -367,7 +367,7 @@ GRT_DEV int bracket_from(const double* axis, int n, double q, int guess) {
 // FP32 polar angle and azimuth of a position in Kerr-Schild coordinates:
 // tan(theta) = sin / cos with sin^2 = (x^2 + y^2) / (r^2 + a^2), cos = z / r.
 // For radii whose squares FP32 holds.
-constexpr double kFp32RadiusMin = 1.0e-12, kFp32RadiusMax = 1.0e12;
+constexpr double kFp32RadiusMax = 1.0e12;
 GRT_DEV void angles_fp32(double a, double x, double y, double z, double r, float& th, float& az) {
     const float rf = static_cast<float>(r), af = static_cast<float>(a);
     th = atan2f(sqrtf(static_cast<float>(x * x + y * y)) * rf, static_cast<float>(z) * sqrtf(rf * rf + af * af));
@@ -392,7 +392,7 @@ constexpr double kAngleMargin = 1.0e-5;
 
 static __device__ __noinline__ int locate_stretched(const KGrid& G, const Axes ax, double a, double x, double y,
                                                     double z, double r) {
-    if (!(r > kFp32RadiusMin && r < kFp32RadiusMax) || G.nr < 2 || G.nth < 2) return kUndecided;
+    if (!(r > G.r_fp32 && r < kFp32RadiusMax) || G.nr < 2 || G.nth < 2) return kUndecided;
     // radius: nearest in the logarithm.  The logarithms' rounding is far
     // inside the margins while the gap is above 1e-6.
     int i;
@@ -458,7 +458,7 @@ static __device__ __noinline__ int locate_stretched(const KGrid& G, const Axes a
 // host asks of the axis -- is left to locate_exact; an edge cell ends within
 // 0.500001 of the spacing, so beyond the margin a position outside is outside.
 GRT_DEV int locate_even(const KGrid& G, double a, double x, double y, double z, double r) {
-    if (!(r > kFp32RadiusMin && r < kFp32RadiusMax)) return kUndecided;
+    if (!(r > G.r_fp32 && r < kFp32RadiusMax)) return kUndecided;
     float th, az;
     angles_fp32(a, x, y, z, r, th, az);
     if (az < 0.0f) az += 6.2831853f;

@@ -34,6 +34,7 @@ struct KGrid {
     // (locate_even; with even = 0 only an index guess, locate_stretched)
     float origin[3], per[3], margin[3];
     int even;
+    double r_fp32;          // radii the FP32 lookups may decide lie beyond it (fp32_lookup_radius)
     double r_certain;       // every cell sampled beyond it has a tetrad (tetrad_certain)
     double r_reject_lo;     // radii outside [lo, hi] cannot pass within_radial_cell
     double r_reject_hi;

@@ -195,6 +195,13 @@ inline void set_axis_lookup(KGrid& g, const double* ra, const double* ta, const 
     g.even = even ? 1 : 0;
 }
 
+// Radius below which the FP32 lookups leave a position to the reference's
+// arithmetic.  The Kerr-Schild radius carries a relative error of about
+// 2^-53 (a / r)^2 and the reference's polar angle acos(z / r) near the axis the
+// root of twice that: at r = a / 100 2e-6, a fifth of the lookups' margins (at a / 2e5
+// ten times them).  Also where FP32 holds the squares.
+inline double fp32_lookup_radius(double a) { return std::fmax(1.0e-12, 0.01 * std::fabs(a)); }
+
 // Stage slots of an RK45 block: the disk mode's rolled error norm keeps the
 // state in a sixth (rk45_attempt).
 __host__ __device__ constexpr int stage_slots(bool disk) { return disk ? 6 : 5; }

@@ -265,6 +265,7 @@ extern "C" grt_status grt_trace_device_noalloc(const grt_params* p, const grt_de
         g.vel_raw = grid->vel4;
         g.mag_raw = grid->mag4;
     }
+    g.r_fp32 = grt::fp32_lookup_radius(p->spin);
     g.r_certain = INFINITY;
     g.vel_scale = p->four_velocity_cm_s_per_code;
     g.mag_scale = p->magnetic_gauss_per_code;

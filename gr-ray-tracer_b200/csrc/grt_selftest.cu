@@ -262,6 +262,7 @@ int grt_selftest_locate(const double* r, int nr, const double* th, int nth, cons
     kp.grid.nph = nph;
     kp.grid.available = kp.grid.separable = 1;
     grt::set_axis_lookup(kp.grid, r, th, ph);
+    kp.grid.r_fp32 = grt::fp32_lookup_radius(spin);
     *is_even = kp.grid.even;
     const grt::dev::Axes ax{da, da + nr, da + nr + nth, da + total, da + total + nr, da + total + nr + nth};
     locate_kernel<<<static_cast<unsigned>((n + 127) / 128), 128>>>(kp, ax, dp, n, d0, d1, d2);
