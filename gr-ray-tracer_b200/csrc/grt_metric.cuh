@@ -91,10 +91,10 @@ GRT_DEV Rhs7 ks_rhs(double x, double y, double z, double pt, double px, double p
     const double dB2 = 2.0 * r * dr2;
     const double dl01 = ((dr0 * x + r) - l1 * dB0) / B;
     const double dl02 = ((dr0 * y - a) - l2 * dB0) / B;
-    const double dl03 = -(l3 * dr0) / r;
+    const double dl03 = (0.0 - l3 * dr0) / r;
     const double dl11 = ((dr1 * x + a) - l1 * dB1) / B;
     const double dl12 = ((dr1 * y + r) - l2 * dB1) / B;
-    const double dl13 = -(l3 * dr1) / r;
+    const double dl13 = (0.0 - l3 * dr1) / r;
     const double dl21 = (dr2 * x - l1 * dB2) / B;
     const double dl22 = (dr2 * y - l2 * dB2) / B;
     const double dl23 = (1.0 - l3 * dr2) / r;
@@ -175,7 +175,8 @@ GRT_DEV double rhs_sqrt_recip(double v, double& recip) {
 // rounds nothing, so x / (2 r) is half of x / r, 4 r^3 d is 2 r^3 (2 d), and a
 // factor left in front of a sum goes into one fma that rounds as the sum does
 // (fma(2, q, u) = RN(u + 2 q)).  d_k = 2 dr/dx^k stands for dr/dx^k, and
-// dH/dx^k is carried halved for k = 0, 1.
+// dH/dx^k is carried halved for k = 0, 1.  Zeros keep their signs: 0 - l3 d is
+// one fma here, which makes +0 of a zero product as the difference does.
 template <bool BF = false>
 GRT_DEV Rhs7 ks_rhs_rcp(double x, double y, double z, double pt, double px, double py, double pz,
                         double a, double M, bool& ok) {
@@ -206,10 +207,10 @@ GRT_DEV Rhs7 ks_rhs_rcp(double x, double y, double z, double pt, double px, doub
     const double dB2 = r * d2;
     const double dl01 = div_by(fma(0.5, d0 * x, r) - l1 * dB0, B, yB);
     const double dl02 = div_by(fma(0.5, d0 * y, -a) - l2 * dB0, B, yB);
-    const double m03 = div_by(l3 * d0, r, yr);  // -2 dl03
+    const double m03 = div_by(fma(-l3, d0, 0.0), r, yr);  // 2 dl03
     const double dl11 = div_by(fma(0.5, d1 * x, a) - l1 * dB1, B, yB);
     const double dl12 = div_by(fma(0.5, d1 * y, r) - l2 * dB1, B, yB);
-    const double m13 = div_by(l3 * d1, r, yr);  // -2 dl13
+    const double m13 = div_by(fma(-l3, d1, 0.0), r, yr);  // 2 dl13
     const double dl21 = div_by(fma(0.5, d2 * x, -(l1 * dB2)), B, yB);
     const double dl22 = div_by(fma(0.5, d2 * y, -(l2 * dB2)), B, yB);
     const double dl23 = div_by(fma(-0.5, l3 * d2, 1.0), r, yr);
@@ -232,8 +233,8 @@ GRT_DEV Rhs7 ks_rhs_rcp(double x, double y, double z, double pt, double px, doub
     o.y = fma(-2.0, H * l2 * ldp, py);
     o.z = fma(-2.0, H * l3 * ldp, pz);
     const double ldp2 = ldp * ldp, two_ldp2 = 2.0 * ldp2;
-    o.px = fma(2.0, Hl * fma(-0.5, m03 * pz, dl01 * px + dl02 * py), h0 * two_ldp2);
-    o.py = fma(2.0, Hl * fma(-0.5, m13 * pz, dl11 * px + dl12 * py), h1 * two_ldp2);
+    o.px = fma(2.0, Hl * fma(0.5, m03 * pz, dl01 * px + dl02 * py), h0 * two_ldp2);
+    o.py = fma(2.0, Hl * fma(0.5, m13 * pz, dl11 * px + dl12 * py), h1 * two_ldp2);
     o.pz = fma(2.0, Hl * ((dl21 * px + dl22 * py) + dl23 * pz), dH2 * ldp2);
     const unsigned small = div_min_nonzero(div_min_nonzero(div_min_nonzero(~0u, x), y), z);
     const unsigned ones = max(max(max(low_word(S), low_word(r)), max(low_word(B), low_word(D))), low_word(DD));
