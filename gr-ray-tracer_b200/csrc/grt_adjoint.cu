@@ -217,7 +217,10 @@ __global__ void __launch_bounds__(128) adj_sweep(const __grid_constant__ KParams
     if (count <= 0) return;
     if (kp.ph.phase[i] != 3) return;  // only ImageArrived rays enter the image
     double lam = dev::pixel_adjoint(kp, aa, i);
-    for (int t = count - 1; t >= 0 && lam != 0.0; --t) {
+    if (lam == 0.0) return;
+    // to the first update, also where lam has become zero: times an infinite
+    // I_before or j0 that is not zero
+    for (int t = count - 1; t >= 0; --t) {
         const double* e = aa.full + static_cast<long long>(t) * dev::kTapeDoubles * n + i;
         lam = dev::sweep_step(kp, aa, lam, static_cast<int>(e[0]), e[n], e[2 * n], e[3 * n], e[4 * n], e[5 * n]);
     }
