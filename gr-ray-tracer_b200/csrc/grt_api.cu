@@ -206,6 +206,7 @@ struct grt_ctx {
     // per-cell multipliers on dtau / dI (differentiable RT)
     DevBuf<double> m_abs, m_emis;
     bool has_m_abs = false, has_m_emis = false;
+    size_t multiplier_cells = 0;
     // checkpointed forward / adjoint
     DevBuf<double> ckpt, tape, dLdI, g_abs, g_emis;
     DevBuf<int> nckpt, adj_overflow, adj_nfull;
@@ -564,6 +565,7 @@ grt_status grt_upload_grid(grt_ctx* c, size_t nr, size_t nth, size_t nph, const 
     c->nr = static_cast<int>(nr);
     c->nth = static_cast<int>(nth);
     c->nph = static_cast<int>(nph);
+    if (ncell != c->multiplier_cells) c->has_m_abs = c->has_m_emis = false;  // those of other cells
     // Separable sorted coordinates -> per-axis binary-search lookup; otherwise
     // the reference's coordinate-descent scans over the full arrays.
     std::vector<double> ra(nr), ta(nth), pa(nph);
@@ -1899,6 +1901,7 @@ grt_status grt_set_cell_multipliers(grt_ctx* c, const double* m_abs, const doubl
     ++c->generation;
     c->adj_ready = false;
     c->has_m_abs = c->has_m_emis = false;
+    c->multiplier_cells = ncell;
     if (m_abs) {
         GRT_CUDA(c, room_for(c, c->m_abs, ncell), "alloc multipliers");
         GRT_CUDA(c, cudaMemcpyAsync(c->m_abs.ptr, m_abs, ncell * sizeof(double), cudaMemcpyDefault, c->stream),

@@ -477,9 +477,11 @@ grt_status grt_render_wait(grt_ctx* ctx, grt_run_stats* stats);
  * dtau = m_abs[cell] * ComputeOpticalDepthIncrement(...) and
  * dI = m_emis[cell] * ComputeEmissivityIncrement(...)
  * (radiative_transfer.hpp:61-96), so the gradient below is exact for any
- * user body.  Arrays are float64 of length nr*ntheta*nphi (C order of
- * the grid), in host memory or on the device (complete when the call is made); NULL switches that multiplier off (all ones).  Applies to every
- * later trace (grt_run, grt_render_graph, the checkpointed forward).
+ * user body.  Arrays are float64 of length nr*ntheta*nphi (C order of the
+ * grid), in host memory or on the device (complete when the call is made);
+ * NULL switches that multiplier off (all ones).  Applies to every later trace
+ * (grt_run, grt_render_graph, the checkpointed forward) until a grid with
+ * another number of cells is uploaded.
  */
 grt_status grt_set_cell_multipliers(grt_ctx* ctx, const double* m_abs, const double* m_emis);
 

@@ -186,6 +186,10 @@ cudaError_t launch_trace(const KParams& kp, bool, int leg, int, int, int blocks_
                 std::to_string(kp.refill_threshold) + " blocks=" + std::to_string(blocks_per_sm) + " order=" + order +
                 (kp.stragglers ? " hands_on" : "") + (kp.resume ? " resume" : "") + "\n";
     if (kp.stragglers && !within(kp.stragglers, kp.n * sizeof(unsigned))) ++bad_accesses;
+    const size_t cells = static_cast<size_t>(kp.grid.nr) * kp.grid.nth * kp.grid.nph;
+    for (const double* m : {kp.m_abs, kp.m_emis})
+        if (m && !within(m, cells * sizeof(double))) ++bad_accesses;
+    if (kp.m_abs || kp.m_emis) launches += "multipliers\n";
     if (leg != 1) kp.counters->terminated = kp.n;
     return cudaSuccess;
 }

@@ -271,3 +271,18 @@ def test_the_tuner_keeps_the_shape_in_force_when_nothing_is_faster(monkeypatch):
     ctx = Tuned()
     best, ms, table = autotune.tune(ctx, lambda c: None, "disk")
     assert best == own == ctx.shape and ms == 1.0 and len(table) == 1 + len(list(autotune.candidates(False)))
+
+
+def test_multipliers_go_with_a_grid_of_other_cells(fake):
+    with lib.Context(image(4)) as ctx:
+        ctx.upload_grid(fluid())
+        ctx.set_cell_multipliers(np.ones(GRID), np.ones(GRID))
+        ctx.upload_grid(fluid())  # as many cells: they stay
+        ctx.init_image_photons(4, 4)
+        ctx.run()
+        assert launches(fake, "multipliers")
+        fake.fake_clear()
+        ctx.upload_grid(torus.benchmark_torus(16, 12, 10, spin=workloads.C2.spin))
+        ctx.init_image_photons(4, 4)
+        ctx.run()
+        assert launches(fake, "trace") and not launches(fake, "multipliers")
