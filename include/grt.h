@@ -140,7 +140,10 @@ typedef struct grt_run_stats {
     uint64_t accepted_steps;    /* ray-steps that advanced a photon */
     uint64_t rejected_attempts; /* RK45 attempts rejected by the controller */
     uint64_t photon_calls;      /* functor invocations on live photons */
-    uint64_t launches;          /* trace-kernel launches issued */
+    uint64_t launches;          /* trace launches: 1 for a chunk of the step loop over whole rays, 3 with
+                                   split legs (backward legs, packet generation, the rest).  A leg's
+                                   second launch, over the rays that its warps handed on, belongs to the
+                                   leg; chunks enqueued past the step the loop stopped at do not count. */
     double trace_ms;            /* device time of the trace launches (CUDA events) */
     int32_t timed_out;          /* 1 if a launch hit its iteration limit */
     int32_t pad;

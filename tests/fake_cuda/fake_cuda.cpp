@@ -137,8 +137,11 @@ cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) {
     launches += "wait\n";
     return cudaSuccess;
 }
-cudaError_t cudaEventCreate(cudaEvent_t* e) { return *e = nullptr, cudaSuccess; }
-cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return *e = nullptr, cudaSuccess; }
+cudaError_t cudaEventCreate(cudaEvent_t* e) {  // any handle that is not null
+    static size_t events = 0;
+    return *e = reinterpret_cast<cudaEvent_t>(++events), cudaSuccess;
+}
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return cudaEventCreate(e); }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaEventRecordWithFlags(cudaEvent_t, cudaStream_t, unsigned) { return cudaSuccess; }

@@ -286,3 +286,26 @@ def test_multipliers_go_with_a_grid_of_other_cells(fake):
         ctx.init_image_photons(4, 4)
         ctx.run()
         assert launches(fake, "trace") and not launches(fake, "multipliers")
+
+
+@pytest.mark.parametrize("way", ["run", "graph", "async"])
+def test_each_leg_hands_on_to_a_second_launch(fake, way):
+    """... which belongs to the leg in the statistics, and comes before what waits for the photons' late fields."""
+    p = image(700)
+    specs = [abi.ImageSpec.from_params(p, 700, 700)]
+    with lib.Context(p) as ctx:
+        ctx.upload_grid(fluid())
+        ctx.init_image_batch(specs)
+        fake.fake_clear()
+        if way == "async":
+            ctx.render_async(abi.PhotonArrays.block(ctx.n), [abi.ProductArrays(700, 700, p.spectrum_bins)])
+            stats = ctx.render_wait()
+        else:
+            stats = ctx.run() if way == "run" else ctx.render_graph()
+    steps = [" ".join(line.split()[:2] + [w for w in line.split() if w in ("hands_on", "resume")])
+             for line in launches(fake)]
+    legs = [s for s in steps if s.startswith("trace") or s == "generate"]
+    assert legs == ["trace 1 hands_on", "trace 1 resume", "generate", "trace 2 hands_on", "trace 2 resume"]
+    assert stats["launches"] == 3
+    if way == "async":
+        assert steps[steps.index("trace 1 resume") + 1] == "wait" and steps.index("wait") < steps.index(legs[0])
