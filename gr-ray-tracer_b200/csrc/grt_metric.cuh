@@ -147,7 +147,8 @@ GRT_DEV Rhs7 ks_rhs(double x, double y, double z, double pt, double px, double p
 // BF selects the branch-free reciprocal and square root of grt_rn.cuh (equal
 // to __drcp_rn and sqrt on every argument that reaches them here: the square
 // roots' results are checked against the box, and every reciprocal's argument
-// lies in [2^-192, 2^164]); without it, CUDA's.
+// lies in [2^-192, 2^164]), as every kernel does; without it CUDA's, which the
+// device self-checks compare with.
 template <bool BF>
 GRT_DEV double rhs_recip(double b) {
     if constexpr (BF) return rcp_rn_core(b);

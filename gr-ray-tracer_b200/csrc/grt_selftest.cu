@@ -2,7 +2,7 @@
 // built into lib/libgrt_selftest.so (test infrastructure; the product library
 // does not link it), with -fmad=false like the trace kernels.
 //   grt_selftest_division  div_by(+-a, |b|, RN(1/|b|)) and IEEE a / b on the same operands;
-//   grt_selftest_rhs       ks_rhs_rcp (and its box flag) and ks_rhs on the same states;
+//   grt_selftest_rhs       ks_rhs_rcp<true>, the kernels' form (and its box flag), and ks_rhs on the same states;
 //   grt_selftest_pow_quarter  the RK45 controller's pow_quarter on the device;
 //   grt_selftest_rn_box    the branch-free reciprocal and square root (grt_rn.cuh)
 //                          and CUDA's __drcp_rn and sqrt on the same arguments;
@@ -36,7 +36,7 @@ __global__ void rhs_kernel(const double* st, size_t n, double spin, double M, do
     if (i >= n) return;
     const double* s = st + 7 * i;
     bool ok = false;
-    const grt::dev::Rhs7 o = grt::dev::ks_rhs_rcp(s[0], s[1], s[2], s[3], s[4], s[5], s[6], spin, M, ok);
+    const grt::dev::Rhs7 o = grt::dev::ks_rhs_rcp<true>(s[0], s[1], s[2], s[3], s[4], s[5], s[6], spin, M, ok);
     const grt::dev::Rhs7 w = grt::dev::ks_rhs(s[0], s[1], s[2], s[3], s[4], s[5], s[6], spin, M);
     const double ov[7] = {o.t, o.x, o.y, o.z, o.px, o.py, o.pz};
     const double wv[7] = {w.t, w.x, w.y, w.z, w.px, w.py, w.pz};

@@ -306,10 +306,10 @@ GRT_DEV void larger_ratio(double& n, double& sc, double m, double sd) {
 // WIDE: the norm's components as straight-line code in registers.  Rolled, its
 // seven chains run one after another through shared memory, a third of a lone
 // warp's attempt.  Trace ms rolled / wide: 256 rays 0.468 / 0.426, adjoint
-// forward of 16,384 rays 1.80 / 1.62, 65,536 rays 1.010 / 0.986, 4.76e6 rays
-// 33.97 / 33.49.  The disk-mode loop, with the sample, transfer and scattering
-// of every step in it, outgrows the instruction cache: 2.07e6 packets 46.1 /
-// 49.1 at 4 blocks/SM, so it stays rolled.
+// forward of 16,384 rays 1.80 / 1.65, 65,536 rays 1.02 / 0.98, 4.76e6 rays
+// 33.9 / 33.7.  The disk-mode loop, with the sample, transfer and scattering
+// of every step in it, outgrows the instruction cache: 2.07e6 packets 45.9 /
+// 50.9 at 4 blocks/SM, so it stays rolled.
 template <class RHS, bool WIDE>
 GRT_DEV int rk45_attempt(const KParams& kp, double s[8], double* dl, int need_k1, int fast, const KStore& kk) {
     const double dt = *dl;
