@@ -368,10 +368,13 @@ GRT_DEV int bracket_from(const double* axis, int n, double q, int guess) {
 // tan(theta) = sin / cos with sin^2 = (x^2 + y^2) / (r^2 + a^2), cos = z / r.
 // For radii whose squares FP32 holds.
 constexpr double kFp32RadiusMax = 1.0e12;
-GRT_DEV void angles_fp32(double a, double x, double y, double z, double r, float& th, float& az) {
+// False so close to the axis that the azimuth's arguments have no FP32 digits.
+GRT_DEV bool angles_fp32(double a, double x, double y, double z, double r, float& th, float& az) {
     const float rf = static_cast<float>(r), af = static_cast<float>(a);
     th = atan2f(sqrtf(static_cast<float>(x * x + y * y)) * rf, static_cast<float>(z) * sqrtf(rf * rf + af * af));
-    az = atan2f(static_cast<float>(r * y - a * x), static_cast<float>(r * x + a * y));
+    const float s = static_cast<float>(r * y - a * x), c = static_cast<float>(r * x + a * y);
+    az = atan2f(s, c);
+    return fmaxf(fabsf(s), fabsf(c)) > 1.0e-30f;
 }
 
 // locate_exact's cell on a separable grid without its logarithms and inverse
@@ -409,7 +412,7 @@ static __device__ __noinline__ int locate_stretched(const KGrid& G, const Axes a
         if (rr > mid) ++i;
     }
     float thf, azf;
-    angles_fp32(a, x, y, z, r, thf, azf);
+    if (!angles_fp32(a, x, y, z, r, thf, azf)) return kUndecided;
     const double th = thf;
     int j;
     if (th < ax.th[0] || th >= ax.th[G.nth - 1]) {
@@ -460,12 +463,12 @@ static __device__ __noinline__ int locate_stretched(const KGrid& G, const Axes a
 GRT_DEV int locate_even(const KGrid& G, double a, double x, double y, double z, double r) {
     if (!(r > G.r_fp32 && r < kFp32RadiusMax)) return kUndecided;
     float th, az;
-    angles_fp32(a, x, y, z, r, th, az);
+    const bool known = angles_fp32(a, x, y, z, r, th, az);
     if (az < 0.0f) az += 6.2831853f;
     const float fi = (logf(static_cast<float>(r)) - G.origin[0]) * G.per[0];
     const float fj = (th - G.origin[1]) * G.per[1], fk = (az - G.origin[2]) * G.per[2];
     const float i = rintf(fi), j = rintf(fj), k = rintf(fk);
-    if (!(fabsf(fi - i) < G.margin[0] && fabsf(fj - j) < G.margin[1] && fabsf(fk - k) < G.margin[2])) return kUndecided;
+    if (!(known && fabsf(fi - i) < G.margin[0] && fabsf(fj - j) < G.margin[1] && fabsf(fk - k) < G.margin[2])) return kUndecided;
     if (i < 0.0f || i > static_cast<float>(G.nr - 1) || j < 0.0f || j > static_cast<float>(G.nth - 1)) return -1;
     int kk = static_cast<int>(k);
     kk += kk < 0 ? G.nph : kk >= G.nph ? -G.nph : 0;
