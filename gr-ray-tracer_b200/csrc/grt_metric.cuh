@@ -175,9 +175,13 @@ GRT_DEV double rhs_sqrt_recip(double v, double& recip) {
 // ks_rhs's tree with its factors of two moved: a product with a power of two
 // rounds nothing, so x / (2 r) is half of x / r, 4 r^3 d is 2 r^3 (2 d), and a
 // factor left in front of a sum goes into one fma that rounds as the sum does
-// (fma(2, q, u) = RN(u + 2 q)).  d_k = 2 dr/dx^k stands for dr/dx^k, and
-// dH/dx^k is carried halved for k = 0, 1.  Zeros keep their signs: 0 - l3 d is
-// one fma here, which makes +0 of a zero product as the difference does.
+// (fma(2, q, u) = RN(u + 2 q)).  d_k = 2 dr/dx^k stands for dr/dx^k; the factor
+// meets it in l3 / 2, and 2 M in place of M makes 2 H and dH/dx^k of the sums.
+// That is for the coordinates, which the box bounds.  The products with the
+// momenta, which nothing bounds (rays that hang at the horizon let them grow to
+// overflow), are ks_rhs's own and overflow where they do.  Zeros keep their
+// signs: 0 - l3 dr is one fma, which makes +0 of a zero product as the
+// difference does.
 template <bool BF = false>
 GRT_DEV Rhs7 ks_rhs_rcp(double x, double y, double z, double pt, double px, double py, double pz,
                         double a, double M, bool& ok) {
@@ -203,40 +207,42 @@ GRT_DEV Rhs7 ks_rhs_rcp(double x, double y, double z, double pt, double px, doub
     const double l1 = div_by(r * x + a * y, B, yB);
     const double l2 = div_by(r * y - a * x, B, yB);
     const double l3 = div_by(z, r, yr);
+    const double hl3 = 0.5 * l3;
     const double dB0 = r * d0;
     const double dB1 = r * d1;
     const double dB2 = r * d2;
     const double dl01 = div_by(fma(0.5, d0 * x, r) - l1 * dB0, B, yB);
     const double dl02 = div_by(fma(0.5, d0 * y, -a) - l2 * dB0, B, yB);
-    const double m03 = div_by(fma(-l3, d0, 0.0), r, yr);  // 2 dl03
+    const double dl03 = div_by(fma(-hl3, d0, 0.0), r, yr);
     const double dl11 = div_by(fma(0.5, d1 * x, a) - l1 * dB1, B, yB);
     const double dl12 = div_by(fma(0.5, d1 * y, r) - l2 * dB1, B, yB);
-    const double m13 = div_by(fma(-l3, d1, 0.0), r, yr);  // 2 dl13
+    const double dl13 = div_by(fma(-hl3, d1, 0.0), r, yr);
     const double dl21 = div_by(fma(0.5, d2 * x, -(l1 * dB2)), B, yB);
     const double dl22 = div_by(fma(0.5, d2 * y, -(l2 * dB2)), B, yB);
-    const double dl23 = div_by(fma(-0.5, l3 * d2, 1.0), r, yr);
+    const double dl23 = div_by(1.0 - hl3 * d2, r, yr);
     const double r3 = r2 * r;
     const double D = r3 * r + az2;
     const double yD = rhs_recip<BF>(D);
-    const double H = div_by(M * r3, D, yD);
+    const double twoM = 2.0 * M;
+    const double twoH = div_by(twoM * r3, D, yD);
     const double three_r2 = 3.0 * r2;
     const double DD = D * D;
     const double yDD = rhs_recip<BF>(DD);
     // dD_k = 2 g_k, and 2 g_2 + 2 a^2 z for k = 2
     const double g0 = r3 * d0, g1 = r3 * d1, g2 = r3 * d2;
-    const double h0 = div_by(M * fma(0.25, three_r2 * d0 * D, -(r3 * g0)), DD, yDD);  // dH0 / 2
-    const double h1 = div_by(M * fma(0.25, three_r2 * d1 * D, -(r3 * g1)), DD, yDD);
+    const double dH0 = div_by(twoM * fma(0.25, three_r2 * d0 * D, -(r3 * g0)), DD, yDD);
+    const double dH1 = div_by(twoM * fma(0.25, three_r2 * d1 * D, -(r3 * g1)), DD, yDD);
     const double dH2 = div_by(M * fma(0.5, three_r2 * d2 * D, -(r3 * fma(2.0, g2, c2))), DD, yDD);
     const double ldp = ((-pt + l1 * px) + l2 * py) + l3 * pz;
-    const double Hl = H * ldp;
-    o.t = fma(2.0, Hl, -pt);
-    o.x = fma(-2.0, H * l1 * ldp, px);
-    o.y = fma(-2.0, H * l2 * ldp, py);
-    o.z = fma(-2.0, H * l3 * ldp, pz);
-    const double ldp2 = ldp * ldp, two_ldp2 = 2.0 * ldp2;
-    o.px = fma(2.0, Hl * fma(0.5, m03 * pz, dl01 * px + dl02 * py), h0 * two_ldp2);
-    o.py = fma(2.0, Hl * fma(0.5, m13 * pz, dl11 * px + dl12 * py), h1 * two_ldp2);
-    o.pz = fma(2.0, Hl * ((dl21 * px + dl22 * py) + dl23 * pz), dH2 * ldp2);
+    const double twoHl = twoH * ldp;
+    o.t = -pt + twoHl;
+    o.x = px - twoH * l1 * ldp;
+    o.y = py - twoH * l2 * ldp;
+    o.z = pz - twoH * l3 * ldp;
+    const double ldp2 = ldp * ldp;
+    o.px = dH0 * ldp2 + twoHl * ((dl01 * px + dl02 * py) + dl03 * pz);
+    o.py = dH1 * ldp2 + twoHl * ((dl11 * px + dl12 * py) + dl13 * pz);
+    o.pz = dH2 * ldp2 + twoHl * ((dl21 * px + dl22 * py) + dl23 * pz);
     const unsigned small = div_min_nonzero(div_min_nonzero(div_min_nonzero(~0u, x), y), z);
     const unsigned ones = max(max(max(low_word(S), low_word(r)), max(low_word(B), low_word(D))), low_word(DD));
     ok = small >= ((1023u - 20u) << 20) - 1u && div_within<-24, 19>(r) && div_within<-60, 41>(S) && ones != ~0u;
