@@ -1,6 +1,7 @@
 """Momenta close to overflow (rays that hang at the horizon when termination.r_min
 lies inside it reach them) and to underflow: the kernels' right-hand side, with
-its factors of two moved, overflows exactly where the reference's expressions do.
+its factors of two moved, and the RK4 step overflow exactly where the
+reference's expressions do.
 
 * ks_rhs_rcp against ks_rhs, bit for bit wherever it does not hand the state on,
   and it keeps every state with momenta of an ordinary size;
@@ -71,3 +72,16 @@ def test_rk45_with_huge_momenta_is_the_oracles(gpu, oracle, spin):
     want, _, wst = run_oracle(oracle, p, grid, photons=ph)
     assert_same_bits(got, want)
     assert gst["accepted_steps"] == wst["accepted_steps"] and (want.terminate == 1).any()
+
+
+@pytest.mark.parametrize("spin", [0.0, 0.94])
+def test_an_rk4_step_overflows_as_the_oracles(gpu, oracle, spin):
+    """2 k2 and 2 k3 overflow by themselves, whatever the sum they go into."""
+    rng = np.random.default_rng(1)
+    w = workloads.ImageWorkload("huge", (16, 8, 8), spin, 60.0, 300, abi.RK4, 0.01, 1)
+    p, grid = w.params().update(camera_distance=100.0, r_term_max=1e6, r_term_min=0.5), w.torus()
+    ph = photons(gpu, p, rng, 300, spin, (2.2, 10.0), rng.uniform(153.5, 154.8, 90000), (0, 1.5))
+    got, _, _ = run_gpu(gpu, p, grid, photons=ph)
+    want, _, _ = run_oracle(oracle, p, grid, photons=ph)
+    assert_same_bits(got, want)
+    assert np.isnan(want.k1).any() and np.isfinite(want.k1).any()
