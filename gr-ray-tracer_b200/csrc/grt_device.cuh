@@ -435,6 +435,9 @@ static __device__ __noinline__ int locate_stretched(const KGrid& G, const Axes a
     if (az < p0 || az >= p1) {
         d = az - p1 + (az < p0 ? 2.0 * kPi : 0.0);
         d2 = p0 - az + (az < p0 ? 0.0 : 2.0 * kPi);
+        // a gap in azimuth: beyond the reach of the cells on both sides
+        if (fmin(d, 2.0 * kPi - d) > ax.phh[k] + kAngleMargin && fmin(d2, 2.0 * kPi - d2) > ax.phh[k2] + kAngleMargin)
+            return -1;
     } else {
         k = bracket_from(ax.ph, n, az, __float2int_rd(static_cast<float>(az - p0) * G.per[2]));
         k2 = k + 1;
