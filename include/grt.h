@@ -170,7 +170,8 @@ typedef struct grt_launch_config {
     int32_t threads_per_block;    /* 128 (the trace kernels' block size) */
     int32_t blocks_per_sm;        /* 2, 3 or 4 resident blocks per SM: register caps 255 / 170 / 128;
                                      0 = automatic: image mode, the fewest that keep every
-                                     geodesic resident; disk mode 2 or 3 by the packet count */
+                                     geodesic resident; disk mode 2 or 3 by the packet count
+                                     (on a grid that is not separable as in image mode) */
     int32_t refill_threshold;     /* idle lanes in a warp before it pulls new photons (1..32) */
     int32_t photons_per_grab;     /* photons a warp claims per access to the global queue; an
                                      image-mode queue is laid out in 8 x 4 pixel tiles, so 32 is
